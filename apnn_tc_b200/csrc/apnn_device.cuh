@@ -41,6 +41,8 @@ struct CoreParams {
   long long out_plane_words;    // packed: words between output bit planes
   const int32_t* residual_in;   // optional dense int32 [rows][N] added before requantisation
   int32_t* residual_out;        // optional dense int32 [rows][N]: the value after the add
+  int* clear_flag;              // optional: a workspace's status flag, which this path has no reason to raise
+  int early_trigger;            // let the next kernel of the stream begin its set-up as soon as this grid is running
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

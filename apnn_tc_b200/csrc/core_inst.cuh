@@ -2,6 +2,7 @@
 // core_wXaY.cu translation units instantiate (one bit-width pair each, so they build in
 // parallel).
 #pragma once
+#include "api_internal.h"
 #include "core_launch.h"
 #include "plane_core.cuh"
 
@@ -21,7 +22,8 @@ template <int AB, int BB>
 using B1Cfg = CoreCfg<KIND_B1, AB, BB, 2, 4, 4, 2, 4>;
 
 template <class Cfg>
-cudaError_t launch_cfg(const CoreParams& p, cudaStream_t stream) {
+cudaError_t launch_cfg(const CoreParams& params, cudaStream_t stream) {
+  CoreParams p = params;
   static bool attr_set[16] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -35,8 +37,16 @@ cudaError_t launch_cfg(const CoreParams& p, cudaStream_t stream) {
   long long tiles_n = ((long long)p.N + Cfg::BN - 1) / Cfg::BN;
   long long grid = tiles_m * tiles_n;
   if (grid <= 0 || grid > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  plane_core_kernel<Cfg><<<(unsigned)grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(p);
-  return cudaGetLastError();
+  p.early_trigger = grid <= 2LL * device_sm_count();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = (unsigned)pdl_attribute(attr);
+  return cudaLaunchKernelEx(&cfg, plane_core_kernel<Cfg>, p);
 }
 
 template <int AB, int BB>

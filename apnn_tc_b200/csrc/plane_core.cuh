@@ -221,6 +221,13 @@ __global__ void __launch_bounds__(Cfg::THREADS) plane_core_kernel(const CorePara
 
   const int ksteps = (p.kchunks + 3) >> 2;
 
+  // Launched as a programmatic dependent: the set-up above overlaps the previous kernel's tail, nothing global is
+  // touched before this wait.  A grid of at most two CTAs per SM lets its own successor start that set-up at once
+  // (the M = 64 problems, whose launch is most of their time); a larger one keeps the SMs to itself.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (p.early_trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.clear_flag != nullptr && blockIdx.x == 0 && tid == 0) *p.clear_flag = 0;
+
 #pragma unroll
   for (int s = 0; s < STAGES - 1; s++) {
     if (s < ksteps) load_stage(s, s);

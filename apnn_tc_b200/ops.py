@@ -25,7 +25,9 @@ from ._cabi import Epilogue
 
 
 def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """cudaStream_t of the current torch stream.  (``torch.cuda.current_stream()`` builds a Stream object on every call,
+    3.2 us of an 11 us launch; the raw handle takes 0.1 us.)"""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _dev_words(t: torch.Tensor, name: str) -> torch.Tensor:
