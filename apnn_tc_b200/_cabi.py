@@ -14,6 +14,7 @@ LIB_PATH = os.path.join(_HERE, "libapnn_b200.so")
 # enums of include/apnn_b200.h
 OUT_INT32, OUT_LOWBITS, OUT_THRESHOLDS, OUT_FLOAT = 0, 1, 2, 3
 QUANT_CENTRED = 0x100   # flag in the `bits` argument of the first-layer int8 gathers
+ROWS_I8, ROWS_FP4 = 1, 2   # Epilogue.out_i8: one byte, or one e2m1 nibble, per output element
 SIGN_NONE, SIGN_W, SIGN_X = 0, 1, 2
 POOL_NONE, POOL_AVG2, POOL_MAX2 = 0, 1, 2
 ALGO_AUTO, ALGO_BMMA, ALGO_IMMA, ALGO_TCGEN05, ALGO_TCGEN05_PAIR = 0, 1, 2, 3, 4
@@ -25,6 +26,7 @@ EXPORTS = (
     "apnn_gemm_workspace_bytes", "apnn_gemm_check", "apnn_expand_planes", "apnn_expand_planes_pair", "apnn_gemm_i8", "apnn_gemm_w8", "apnn_expand_planes_fp4", "apnn_gemm_fp4", "apnn_gemm_static_scratch", "apnn_conv2d", "apnn_conv2d_ex",
     "apnn_conv2d_workspace_bytes", "apnn_conv2d_check", "apnn_conv2d_i8", "apnn_bit_compress", "apnn_quantize_pack", "apnn_quantize_im2col", "apnn_create",
     "apnn_destroy", "apnn_gemm_host", "apnn_conv2d_host", "apnn_probe_peak", "apnn_quantize_im2col_i8", "apnn_quantize_window_rows_i8", "apnn_quantize_blocks_i8", "apnn_maxpool2x2_i8", "apnn_requantize_i32",
+    "apnn_conv2d_fp4", "apnn_conv2d_i8_to_fp4", "apnn_maxpool2x2_rows",
 )
 
 
@@ -103,6 +105,9 @@ def lib() -> ctypes.CDLL:
     L.apnn_quantize_window_rows_i8.argtypes = [vp, vp, vp, i, i, i, i, i, i, i, i]
     L.apnn_quantize_blocks_i8.argtypes = [vp, vp, vp, i, i, i, i, i, i, i, i]
     L.apnn_maxpool2x2_i8.argtypes = [vp, vp, vp, i, i, i, i, i, i]
+    L.apnn_conv2d_i8_to_fp4.argtypes = L.apnn_conv2d_i8.argtypes
+    L.apnn_conv2d_fp4.argtypes = [vp, vp, vp, vp, i, i, i, i, i, i, ep, vp]
+    L.apnn_maxpool2x2_rows.argtypes = [vp, vp, vp, i, i, i, i, i, i, i, i]
     L.apnn_requantize_i32.argtypes = [vp, vp, vp, ctypes.c_long, i, vp]
     L.apnn_create.argtypes = [ctypes.POINTER(vp), i]
     L.apnn_destroy.argtypes = [vp]

@@ -38,13 +38,15 @@ int device_sm_count() {
 }
 
 apnn_status check_epilogue(const apnn_epilogue* e, int channels, bool is_conv, int abits_signed_w, int abits_signed_x,
-                           bool i8_rows_ok) {
+                           bool i8_rows_ok, bool fp4_rows_ok) {
   if (!e) return APNN_OK;
   if (e->struct_size != sizeof(apnn_epilogue)) return APNN_ERR_INVALID_ARG;   // built against another layout
   if (e->residual_i16 != 0 && (e->residual_i16 < 0 || e->residual_i16 > 3 || !i8_rows_ok || e->n_peer_out != 0))
     return (e->residual_i16 > 0 && e->residual_i16 <= 3 && !i8_rows_ok) ? APNN_ERR_UNSUPPORTED : APNN_ERR_INVALID_ARG;
-  if (e->out_i8 != 0 && (e->out_i8 != 1 || !i8_rows_ok || e->out_mode == APNN_OUT_INT32 || e->n_peer_out != 0))
+  const bool rows_form = e->out_i8 == 1 || (e->out_i8 == APNN_ROWS_FP4 && fp4_rows_ok);
+  if (e->out_i8 != 0 && (!rows_form || !i8_rows_ok || e->out_mode == APNN_OUT_INT32 || e->n_peer_out != 0))
     return e->out_i8 == 1 && !i8_rows_ok ? APNN_ERR_UNSUPPORTED : APNN_ERR_INVALID_ARG;
+  if (e->out_i8 == APNN_ROWS_FP4 && e->out_bits > 2) return APNN_ERR_UNSUPPORTED;   // 5, 6, 7 are not e2m1 values
   if (e->out_mode < APNN_OUT_INT32 || e->out_mode > APNN_OUT_FLOAT) return APNN_ERR_INVALID_ARG;
   if (e->out_mode == APNN_OUT_FLOAT) {
     // the float affine exists in the tcgen05 kernels' run-time epilogue and in apnn_requantize_i32
@@ -298,15 +300,16 @@ apnn_status apnn_conv2d_check(void* stream, const void* workspace, int B, int H,
   return flag == 0 ? APNN_OK : APNN_ERR_TIMEOUT;
 }
 
-apnn_status apnn_conv2d_i8(void* stream, const void* W8, const void* X8, void* Out, int B, int H, int W, int CIN,
-                           int COUT, int R, int stride, int w_signed, const apnn_epilogue* epi, int* status_flag) {
+static apnn_status conv2d_i8(void* stream, const void* W8, const void* X8, void* Out, int B, int H, int W, int CIN,
+                             int COUT, int R, int stride, int w_signed, const apnn_epilogue* epi, int* status_flag,
+                             bool fp4_rows) {
   if (!W8 || !X8 || !Out || !status_flag) return APNN_ERR_INVALID_ARG;
   if (B <= 0 || H <= 0 || W <= 0 || CIN <= 0 || COUT <= 0) return APNN_ERR_INVALID_ARG;
   if (R < 1 || R > 11 || (R & 1) == 0) return APNN_ERR_UNSUPPORTED;
   if (CIN % 64 != 0 || !aligned16(W8) || !aligned16(X8) || !aligned16(Out)) return APNN_ERR_ALIGNMENT;
   if (epi) {
     if (epi->signed_operand != APNN_SIGN_NONE) return APNN_ERR_INVALID_ARG;  // the sign is in the bytes
-    apnn_status st = check_epilogue(epi, COUT, true, 1, 1, true);
+    apnn_status st = check_epilogue(epi, COUT, true, 1, 1, true, fp4_rows);
     if (st == APNN_OK && epi->out_i8 && !aligned32(Out)) st = APNN_ERR_ALIGNMENT;
     if (st != APNN_OK) return st;
     if (epi->pool != APNN_POOL_NONE && ((((H - 1) / (stride > 0 ? stride : 1) + 1) & 1) ||
@@ -318,6 +321,40 @@ apnn_status apnn_conv2d_i8(void* stream, const void* W8, const void* X8, void* O
   if (w_signed < 0 || w_signed > 3) return APNN_ERR_INVALID_ARG;
   return tc5_conv_i8(reinterpret_cast<cudaStream_t>(stream), (const uint8_t*)X8, (const uint8_t*)W8, Out, B, H, W,
                      CIN, COUT, R, stride, (w_signed & 1) != 0, epi, status_flag, (w_signed & 2) != 0);
+}
+
+apnn_status apnn_conv2d_i8(void* stream, const void* W8, const void* X8, void* Out, int B, int H, int W, int CIN,
+                           int COUT, int R, int stride, int w_signed, const apnn_epilogue* epi, int* status_flag) {
+  return conv2d_i8(stream, W8, X8, Out, B, H, W, CIN, COUT, R, stride, w_signed, epi, status_flag, false);
+}
+
+apnn_status apnn_conv2d_i8_to_fp4(void* stream, const void* W8, const void* X8, void* Out, int B, int H, int W, int CIN,
+                                  int COUT, int R, int stride, int w_signed, const apnn_epilogue* epi, int* status_flag) {
+  if (!epi || epi->out_i8 != APNN_ROWS_FP4) return APNN_ERR_INVALID_ARG;
+  return conv2d_i8(stream, W8, X8, Out, B, H, W, CIN, COUT, R, stride, w_signed, epi, status_flag, true);
+}
+
+apnn_status apnn_conv2d_fp4(void* stream, const void* W4, const void* X4, void* Out, int B, int H, int W, int CIN, int COUT,
+                            int R, const apnn_epilogue* epi, int* status_flag) {
+  if (!W4 || !X4 || !Out || !status_flag) return APNN_ERR_INVALID_ARG;
+  if (B <= 0 || H <= 0 || W <= 0 || CIN <= 0 || COUT <= 0) return APNN_ERR_INVALID_ARG;
+  if (R != 1 && R != 3) return APNN_ERR_UNSUPPORTED;
+  if (CIN % 128 != 0 || !aligned16(W4) || !aligned16(X4) || !aligned16(Out)) return APNN_ERR_ALIGNMENT;
+  const int pad = (R - 1) / 2;
+  int in_halo = pad, out_halo = 0;
+  if (epi) {
+    if (epi->signed_operand != APNN_SIGN_NONE) return APNN_ERR_INVALID_ARG;  // the sign is in the nibbles
+    apnn_status st = check_epilogue(epi, COUT, true, 1, 1, true, true);
+    if (st == APNN_OK && epi->out_i8 == 1 && !aligned32(Out)) st = APNN_ERR_ALIGNMENT;
+    if (st != APNN_OK) return st;
+    if (epi->pool != APNN_POOL_NONE || epi->out_mode == APNN_OUT_FLOAT) return APNN_ERR_UNSUPPORTED;
+    if (epi->in_halo != 0 && epi->in_halo < pad) return APNN_ERR_INVALID_ARG;
+    if (epi->in_halo != 0) in_halo = epi->in_halo;
+    out_halo = epi->out_halo;
+  }
+  if (tc5_conv_fp4_clocks(B, H, W, CIN, COUT, R, in_halo, out_halo) == 0) return APNN_ERR_UNSUPPORTED;
+  return tc5_conv_fp4(reinterpret_cast<cudaStream_t>(stream), (const uint8_t*)X4, (const uint8_t*)W4, Out, B, H, W, CIN, COUT,
+                      R, epi, status_flag);
 }
 
 apnn_status apnn_conv2d(void* stream, int wbits, int xbits, const void* Wt, const void* X, void* Out, int B, int H,

@@ -9,7 +9,7 @@ apnn_status cuda_fail(cudaError_t e, const char* where);
 int device_sm_count();
 // Validates an epilogue descriptor; wbits/xbits are the widths of the W and X arguments.
 apnn_status check_epilogue(const apnn_epilogue* e, int channels, bool is_conv, int wbits, int xbits,
-                           bool i8_rows_ok = false);
+                           bool i8_rows_ok = false, bool fp4_rows_ok = false);
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel, device); safe to call from several threads.
 cudaError_t ensure_max_smem(const void* kernel, int bytes);
 // Address of the driver's cuTensorMapEncodeTiled (null if unavailable); looked up once, thread-safe.

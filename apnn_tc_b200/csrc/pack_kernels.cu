@@ -643,6 +643,59 @@ __global__ void __launch_bounds__(256) maxpool2x2_i8_kernel(const uint8_t* __res
   }
 }
 
+// Four level bytes 0..3 -> their e2m1 codes 0, 2, 4, 5 (one per byte).
+__device__ __forceinline__ uint32_t e2m1_codes4(uint32_t lv) { return (lv << 1) - (lv & (lv >> 1) & 0x01010101u); }
+
+// The same pass with e2m1 nibble rows on the output side, and on the input side too when FP4_IN.  A thread owns 32
+// channels of an output pixel: one 16-byte store.  Byte 4q + i of an int8 group and nibble 2i + (q >> 2) of nibble word
+// q & 3 hold the same element, so a nibble word is two words of codes merged.
+template <bool FP4_IN>
+__global__ void __launch_bounds__(256) maxpool2x2_fp4_kernel(const uint8_t* __restrict__ in, uint8_t* __restrict__ out, int B,
+                                                             int Ho, int Wo, int C, int ih, int oh) {
+  const int groups = C >> 5;
+  const uint32_t total = (uint32_t)B * Ho * Wo * groups;   // the host checks that it fits
+  const int Wi = 2 * Wo + 2 * ih, Hi = 2 * Ho + 2 * ih, Wq = Wo + 2 * oh, Hq = Ho + 2 * oh;
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // launched as a programmatic dependent of the producing layer
+  constexpr int V = FP4_IN ? 1 : 2;   // 16-byte vectors of a group in one input pixel
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
+    const uint32_t pix = t / (uint32_t)groups;
+    const int g = (int)(t - pix * groups);
+    const uint32_t rowi = pix / (uint32_t)Wo;
+    const int wo = (int)(pix - rowi * Wo);
+    const int b = (int)(rowi / (uint32_t)Ho), ho = (int)(rowi - (uint32_t)b * Ho);
+    const long long p0 = ((long long)b * Hi + 2 * ho + ih) * Wi + 2 * wo + ih;
+    const int pv = groups * V;   // vectors per input pixel
+    const uint4* src = reinterpret_cast<const uint4*>(in) + p0 * pv + g * V;
+    uint4 x[4][V];
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+      x[0][v] = __ldg(src + v);
+      x[1][v] = __ldg(src + pv + v);
+      x[2][v] = __ldg(src + (long long)Wi * pv + v);
+      x[3][v] = __ldg(src + (long long)Wi * pv + pv + v);
+    }
+    auto max4 = [](uint32_t a, uint32_t c, uint32_t d, uint32_t e) { return __vmaxu4(__vmaxu4(a, c), __vmaxu4(d, e)); };
+    uint32_t o[4];
+    if constexpr (FP4_IN) {
+      auto both = [&](uint32_t a, uint32_t c, uint32_t d, uint32_t e) {
+        constexpr uint32_t L = 0x0F0F0F0Fu;
+        return max4(a & L, c & L, d & L, e & L) | max4(a & ~L, c & ~L, d & ~L, e & ~L);
+      };
+      o[0] = both(x[0][0].x, x[1][0].x, x[2][0].x, x[3][0].x);
+      o[1] = both(x[0][0].y, x[1][0].y, x[2][0].y, x[3][0].y);
+      o[2] = both(x[0][0].z, x[1][0].z, x[2][0].z, x[3][0].z);
+      o[3] = both(x[0][0].w, x[1][0].w, x[2][0].w, x[3][0].w);
+    } else {
+      constexpr int H1 = V - 1;
+      o[0] = e2m1_codes4(max4(x[0][0].x, x[1][0].x, x[2][0].x, x[3][0].x)) | (e2m1_codes4(max4(x[0][H1].x, x[1][H1].x, x[2][H1].x, x[3][H1].x)) << 4);
+      o[1] = e2m1_codes4(max4(x[0][0].y, x[1][0].y, x[2][0].y, x[3][0].y)) | (e2m1_codes4(max4(x[0][H1].y, x[1][H1].y, x[2][H1].y, x[3][H1].y)) << 4);
+      o[2] = e2m1_codes4(max4(x[0][0].z, x[1][0].z, x[2][0].z, x[3][0].z)) | (e2m1_codes4(max4(x[0][H1].z, x[1][H1].z, x[2][H1].z, x[3][H1].z)) << 4);
+      o[3] = e2m1_codes4(max4(x[0][0].w, x[1][0].w, x[2][0].w, x[3][0].w)) | (e2m1_codes4(max4(x[0][H1].w, x[1][H1].w, x[2][H1].w, x[3][H1].w)) << 4);
+    }
+    reinterpret_cast<uint4*>(out)[(((long long)b * Hq + ho + oh) * Wq + wo + oh) * groups + g] = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 // First layer with a stride: the image regrouped into stride x stride pixel blocks ("space to depth").  Block
 // (hb, wb) of image b becomes one pixel of cpad bytes, byte (di*stride + dj)*C + c = level of pixel
 // (stride*hb + di, stride*wb + dj), channel c; bytes from stride*stride*C on are 0.  The strided RxR convolution of
@@ -960,6 +1013,35 @@ apnn_status apnn_maxpool2x2_i8(void* stream, const void* in_i8, void* out_i8, in
   cudaError_t e = cudaLaunchKernelEx(&cfg, maxpool2x2_i8_kernel, reinterpret_cast<const uint8_t*>(in_i8),
                                      reinterpret_cast<uint8_t*>(out_i8), B, H / 2, W / 2, C, in_halo, out_halo);
   if (e != cudaSuccess) return cuda_fail(e, "maxpool2x2_i8 launch");
+  return APNN_OK;
+}
+
+apnn_status apnn_maxpool2x2_rows(void* stream, const void* in, void* out, int B, int H, int W, int C, int in_halo, int out_halo,
+                                 int in_form, int out_form) {
+  using namespace apnn;
+  if (in_form == 1 && out_form == 1) return apnn_maxpool2x2_i8(stream, in, out, B, H, W, C, in_halo, out_halo);
+  if (!in || !out || B <= 0 || H <= 0 || W <= 0 || C <= 0) return APNN_ERR_INVALID_ARG;
+  if ((in_form != 1 && in_form != APNN_ROWS_FP4) || (out_form != 1 && out_form != APNN_ROWS_FP4)) return APNN_ERR_INVALID_ARG;
+  if (in_halo < 0 || in_halo > 8 || out_halo < 0 || out_halo > 8) return APNN_ERR_INVALID_ARG;
+  if ((H & 1) || (W & 1) || out_form != APNN_ROWS_FP4) return APNN_ERR_UNSUPPORTED;
+  if (C % 32 != 0 || (reinterpret_cast<uintptr_t>(in) & 15u) || (reinterpret_cast<uintptr_t>(out) & 15u))
+    return APNN_ERR_ALIGNMENT;
+  const long long total = (long long)B * (H / 2) * (W / 2) * (C / 32);
+  long long nb = (total + 255) / 256, cap = (long long)device_sm_count() * 32;
+  if (nb > cap) nb = cap;
+  if (total + nb * 256 > 0xffffffffLL) return APNN_ERR_UNSUPPORTED;   // 32-bit indices
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)nb, 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = reinterpret_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = (unsigned)pdl_attribute(attr);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, in_form == 1 ? maxpool2x2_fp4_kernel<false> : maxpool2x2_fp4_kernel<true>,
+                                     reinterpret_cast<const uint8_t*>(in), reinterpret_cast<uint8_t*>(out), B, H / 2, W / 2, C,
+                                     in_halo, out_halo);
+  if (e != cudaSuccess) return cuda_fail(e, "maxpool2x2_rows launch");
   return APNN_OK;
 }
 

@@ -341,7 +341,7 @@ bool tc5_conv_pair_applies(int B, int Hin, int Win, int CIN, int COUT, int R, in
   static const bool disabled = [] { const char* v = getenv("APNN_CONV_PAIR"); return v && v[0] == '0'; }();
   if (disabled) return false;
   if (!epi || stride != 1 || CIN % 128 != 0 || COUT % TILE_N != 0 || (R != 1 && R != 3)) return false;
-  if (epi->pool != APNN_POOL_NONE || epi->out_mode != APNN_OUT_THRESHOLDS || !epi->out_i8 || !epi->thresholds) return false;
+  if (epi->pool != APNN_POOL_NONE || epi->out_mode != APNN_OUT_THRESHOLDS || epi->out_i8 != 1 || !epi->thresholds) return false;
   if (epi->out_bits != 1 && epi->out_bits != 2) return false;
   if (epi->residual_in || epi->residual_out || epi->n_peer_out) return false;
   const int pad = (R - 1) / 2;

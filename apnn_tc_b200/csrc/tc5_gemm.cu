@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(256) expand_planes_kernel(const ExpandJob a, c
   const long long blk = first ? blockIdx.x : blockIdx.x - blocks_a;
   const long long i0 = blk * blockDim.x + threadIdx.x;
   const long long step = nblk * blockDim.x;
+  tc5::grid_dependency_wait();   // launched as a programmatic dependent: nothing global is touched before this
   switch (j.bits) {
     case 1: expand_words<1>(j, i0, step); break;
     case 2: expand_words<2>(j, i0, step); break;
@@ -142,7 +143,7 @@ struct Tc5Params {
   int M, N, kblocks;
   int tiles_m, tiles_n;
   int out_mode, out_bits;
-  int out_i8;            // quantised outputs as one byte per element (rows of N bytes) instead of packed planes
+  int out_i8;            // quantised outputs as one byte (1: rows of N bytes) or one e2m1 nibble (2) per element, not packed planes
   uint32_t idesc;
   long long out_plane_words;
   int* error_flag;
@@ -241,6 +242,14 @@ __device__ __forceinline__ RowDst row_destination(const Tc5Params& p, int tm, in
   d.row = ((long long)b * (p.out_h + 2 * hh) + oh + hh) * (p.out_w + 2 * hh) + ow + hh;
   d.dense = ((long long)b * p.out_h + oh) * p.out_w + ow;
   return d;
+}
+
+// The 32 level bytes of an int8 group -> its 16 bytes of e2m1 nibbles (codes 0, 2, 4, 5 of the levels 0..3): byte i of
+// word q becomes nibble 2i + (q >> 2) of nibble word q & 3.
+__device__ __forceinline__ uint4 nibble_group(const uint32_t (&r)[8]) {
+  auto codes = [](uint32_t lv) { return (lv << 1) - (lv & (lv >> 1) & 0x01010101u); };
+  return make_uint4(codes(r[0]) | (codes(r[4]) << 4), codes(r[1]) | (codes(r[5]) << 4), codes(r[2]) | (codes(r[6]) << 4),
+                    codes(r[3]) | (codes(r[7]) << 4));
 }
 
 __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, int& tm, int& tn) {
@@ -416,6 +425,7 @@ __device__ __forceinline__ bool flat_issue_taps_ring(uint32_t d_tmem, uint32_t a
 //   3  as 2 plus residual in / out of either width (second convolution of a ResNet block)
 //   4  as 3 with every residual tensor present being int16 (no int32 residual code)
 //   5  int32 output only (shortcut convolutions, logits)
+//   6, 7  as 2 and 3, but e2m1 nibble rows (the layer in front of a 4-bit convolution)
 //
 // SPLITK: the kernel is launched as clusters of p.splits CTAs (2, 4 or 8) with one output tile per
 // cluster, for problems with fewer tiles than SMs and a long K.  CTA r of a cluster accumulates K
@@ -743,8 +753,10 @@ tc5_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else {
     // ---------------- epilogue warps (2..9) ----------------
-    constexpr bool C_NOPOOL = EPI >= 1, C_NORES = EPI == 1 || EPI == 2 || EPI == 5, C_NOINT32 = EPI >= 1 && EPI <= 4;
-    constexpr bool C_I8THR = EPI >= 2 && EPI <= 4, C_RES16 = EPI == 4, C_INT32 = EPI == 5;
+    constexpr bool C_NOPOOL = EPI >= 1, C_NORES = EPI == 1 || EPI == 2 || EPI == 5 || EPI == 6, C_NOINT32 = EPI >= 1 && EPI != 5;
+    constexpr bool C_I8THR = (EPI >= 2 && EPI <= 4) || EPI >= 6, C_RES16 = EPI == 4, C_INT32 = EPI == 5;
+    // nibble rows: epilogues of their own, or the run-time one (a branch in the others made the 64-channel layers 1 % slower)
+    const bool NIBBLES = EPI >= 6 || (EPI == 0 && p.out_i8 == 2);
     grid_dependency_wait();   // residual reads and every store of this kernel come after this
     const int ew = warp - 2;
     const int quarter = warp & 3;  // TMEM lanes 32*quarter .. +31 are the ones this warp may read
@@ -1081,6 +1093,10 @@ tc5_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               if (x >= q4.y) r[(31 - j) & 7] += inc;
               if (x >= q4.z) r[(31 - j) & 7] += inc;
             }
+            if (NIBBLES) {
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + ((row * p.N + col0) >> 1)) = nibble_group(r);
+              continue;
+            }
             uint8_t* O8 = reinterpret_cast<uint8_t*>(p.out) + row * p.N + col0;
             asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(O8), "r"(r[0]), "r"(r[1]), "r"(r[2]),
                          "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -1114,6 +1130,10 @@ tc5_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             uint32_t r[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll
             for (int j = 0; j < 32; j++) r[(31 - j) & 7] |= lv[j] << (8 * ((31 - j) >> 3));
+            if (NIBBLES) {
+              *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + ((row * p.N + col0) >> 1)) = nibble_group(r);
+              continue;
+            }
             uint8_t* O8 = reinterpret_cast<uint8_t*>(p.out) + row * p.N + col0;
             asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(O8), "r"(r[0]), "r"(r[1]), "r"(r[2]),
                          "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -1329,9 +1349,12 @@ cudaError_t launch_tc5_p(cudaStream_t s, const CUtensorMap& map_a, const CUtenso
   const bool thr_i8 = p.out_mode == APNN_OUT_THRESHOLDS && p.out_bits <= 2 && p.out_i8;
   const bool all16 = (!p.residual_in || p.res16_in) && (!p.residual_out || p.res16_out);
   const bool int32_only = p.out_mode == APNN_OUT_INT32 && p.pool == APNN_POOL_NONE && !residuals;
-  const int epi = int32_only ? 5 : !quantising ? 0 : (thr_i8 ? (residuals ? (all16 ? 4 : 3) : 2) : (residuals ? 0 : 1));
+  const bool thr_fp4 = p.out_mode == APNN_OUT_THRESHOLDS && p.out_bits <= 2 && p.out_i8 == 2;
+  const int epi = int32_only ? 5 : !quantising ? 0 : p.out_i8 == 2 ? (thr_fp4 ? (residuals ? 7 : 6) : 0) : (thr_i8 ? (residuals ? (all16 ? 4 : 3) : 2) : (residuals ? 0 : 1));
   if (epi == 1) return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 1, PAIR>, s, grid, smem, pair_ctas, map_a, map_b, p);
   if constexpr (!PAIR) {
+    if (epi == 6 && p.is_conv == 2 && p.R == 5)
+      return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 6, false, true>, s, grid, smem, pair_ctas, map_a, map_b, p);
     if (epi == 2 && p.is_conv == 2 && p.R == 5)
       return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 2, false, true>, s, grid, smem, pair_ctas, map_a, map_b, p);
   }
@@ -1339,6 +1362,8 @@ cudaError_t launch_tc5_p(cudaStream_t s, const CUtensorMap& map_a, const CUtenso
   if (epi == 3) return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 3, PAIR>, s, grid, smem, pair_ctas, map_a, map_b, p);
   if (epi == 4) return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 4, PAIR>, s, grid, smem, pair_ctas, map_a, map_b, p);
   if (epi == 5) return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 5, PAIR>, s, grid, smem, pair_ctas, map_a, map_b, p);
+  if (epi == 6) return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 6, PAIR>, s, grid, smem, pair_ctas, map_a, map_b, p);
+  if (epi == 7) return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 7, PAIR>, s, grid, smem, pair_ctas, map_a, map_b, p);
   return launch_kernel(tc5_gemm_kernel<BN, BKB, false, 0, PAIR>, s, grid, smem, pair_ctas, map_a, map_b, p);
 }
 
@@ -1499,28 +1524,33 @@ ExpandJob make_job(const uint32_t* planes, uint8_t* out, long long rows, int K, 
 // the ABI only admits 1..4 and 8
 }  // namespace
 
-apnn_status tc5_expand(cudaStream_t s, const uint32_t* planes, uint8_t* out, long long rows, int K, int bits,
-                       bool is_signed) {
-  const int sms = device_sm_count();
-  ExpandJob a = make_job(planes, out, rows, K, bits, is_signed);
-  const int blocks = expand_blocks(a.total, sms);
-  expand_planes_kernel<<<blocks, 256, 0, s>>>(a, a, blocks);
-  cudaError_t e = cudaGetLastError();
+static apnn_status launch_expand(cudaStream_t s, const ExpandJob& a, const ExpandJob& b, int ba, int bb) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(ba + bb), 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = (unsigned)pdl_attribute(attr);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, expand_planes_kernel, a, b, ba);
   if (e != cudaSuccess) return cuda_fail(e, "expand_planes launch");
   return APNN_OK;
 }
 
-// Both operands of a GEMM in one launch.
+apnn_status tc5_expand(cudaStream_t s, const uint32_t* planes, uint8_t* out, long long rows, int K, int bits,
+                       bool is_signed) {
+  ExpandJob a = make_job(planes, out, rows, K, bits, is_signed);
+  return launch_expand(s, a, a, expand_blocks(a.total, device_sm_count()), 0);
+}
+
+// Both operands of a GEMM or a convolution in one launch (rows x K only counts words: planes and bytes are linear).
 apnn_status tc5_expand2(cudaStream_t s, const uint32_t* pa, uint8_t* oa, long long rows_a, int bits_a, bool signed_a,
                         const uint32_t* pb, uint8_t* ob, long long rows_b, int bits_b, bool signed_b, int K) {
   const int sms = device_sm_count();
   ExpandJob a = make_job(pa, oa, rows_a, K, bits_a, signed_a);
   ExpandJob b = make_job(pb, ob, rows_b, K, bits_b, signed_b);
-  const int ba = expand_blocks(a.total, sms), bb = expand_blocks(b.total, sms);
-  expand_planes_kernel<<<ba + bb, 256, 0, s>>>(a, b, ba);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "expand_planes launch");
-  return APNN_OK;
+  return launch_expand(s, a, b, expand_blocks(a.total, sms), expand_blocks(b.total, sms));
 }
 
 // Problems the 256 x 256 CTA-pair kernel takes: enough tiles for every SM pair (or peer destinations, which only
@@ -1599,8 +1629,7 @@ apnn_status tc5_gemm(cudaStream_t s, int wbits, int xbits, const uint32_t* W, co
   if (fp4_on && wbits <= 2 && xbits <= 2 && K % 256 == 0 && (long long)K * 9 < (1ll << 24) &&
       (pair || takes_pair_kernel(M, N, K, epi)) && !(epi && epi->out_mode == APNN_OUT_FLOAT)) {
     uint8_t* xb4 = wa + align_up((size_t)M * (K / 2), 256);
-    apnn_status s4 = tc5_expand_fp4(s, W, wa, M, K, wbits, sign == APNN_SIGN_W);
-    if (s4 == APNN_OK) s4 = tc5_expand_fp4(s, X, xb4, N, K, xbits, sign == APNN_SIGN_X);
+    apnn_status s4 = tc5_expand2_fp4(s, W, wa, M, wbits, sign == APNN_SIGN_W, X, xb4, N, xbits, sign == APNN_SIGN_X, K);
     if (s4 != APNN_OK) return s4;
     return tc5_gemm_fp4_pair(s, wa, xb4, D, M, N, K, epi, err);
   }
@@ -1792,9 +1821,22 @@ apnn_status tc5_conv(cudaStream_t s, int wbits, int xbits, const uint32_t* Wt, c
   uint8_t* w8 = x8 + align_up((size_t)pixels * CIN, 256);
   int* err = reinterpret_cast<int*>(w8 + align_up((size_t)COUT * R * R * CIN, 256));
   const bool w_signed = epi && epi->signed_operand == APNN_SIGN_W;
-  apnn_status st = tc5_expand(s, X, x8, pixels, CIN, xbits, false);
-  if (st != APNN_OK) return st;
-  st = tc5_expand(s, Wt, w8, COUT, R * R * CIN, wbits, w_signed);
+  // Operands of at most two bits as e2m1 nibbles where the flat 4-bit convolution takes the shape: half the bytes to
+  // write and read, twice the tensor rate.  (Filter rows are counted in 128-channel rows: planes and nibbles are linear.)
+  // Its tiles are 256 channels wide, so it needs more than 64 (32 x 28x28, 128 -> 64 channels: 13.4 us against 12.6 on
+  // int8; 128 -> 96 and 128 -> 128: 10.1 / 13.5 against 10.4 / 13.9), and outside the two-bit thresholds its general
+  // epilogue needs some K to hide behind (int32, 32 x 28x28, 128 -> 128: 17.2 against 12.9; 256 -> 160: 18.8 against 20.5).
+  const bool thr2 = epi && epi->out_mode == APNN_OUT_THRESHOLDS && epi->out_bits <= 2 && !epi->residual_in && !epi->residual_out;
+  static const bool fp4_on = [] { const char* v = getenv("APNN_FP4"); return !(v && v[0] == '0'); }();
+  if (fp4_on && wbits <= 2 && xbits <= 2 && stride == 1 && CIN % 128 == 0 && COUT > 64 && (thr2 || R * R * CIN >= 2048) && (!epi || epi->pool == APNN_POOL_NONE) &&
+      tc5_conv_fp4_clocks(B, H, W, CIN, COUT, R, pad, epi ? epi->out_halo : 0) != 0) {
+    apnn_status s4 = tc5_expand2_fp4(s, X, x8, pixels * (CIN / 128), xbits, false, Wt, w8, (long long)COUT * R * R * (CIN / 128),
+                                     wbits, w_signed, 128);
+    if (s4 != APNN_OK) return s4;
+    return tc5_conv_fp4(s, x8, w8, Out, B, H, W, CIN, COUT, R, epi, err);
+  }
+  apnn_status st = tc5_expand2(s, X, x8, pixels * (CIN / 64), xbits, false, Wt, w8, (long long)COUT * R * R * (CIN / 64), wbits,
+                               w_signed, 64);
   if (st != APNN_OK) return st;
   return tc5_conv_i8(s, x8, w8, Out, B, H, W, CIN, COUT, R, stride, w_signed, epi, err);
 }

@@ -667,12 +667,26 @@ tc5_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // two planes (0 -> 0000, 1 -> 0010, 2 -> 0100, 3 -> 0101), or -1 / +1 of a single plane (bit 0 -> 1010, 1 -> 0010).
 // Nibble i of output word q holds the element whose bit sits at position 4*i + q: a fixed permutation inside each
 // group of 32 k, the same for both operands.
-__global__ void __launch_bounds__(256) expand_nibbles_kernel(const uint32_t* __restrict__ planes, uint8_t* __restrict__ out,
-                                                             long long total, int bits, int is_signed) {
+struct NibbleJob {
+  const uint32_t* planes;
+  uint8_t* out;
+  long long total;   // words per plane
+  int bits, is_signed;
+};
+// Blocks [0, blocks_a) work on job a, the rest on job b: both operands of a contraction in one launch.
+__global__ void __launch_bounds__(256) expand_nibbles_kernel(const NibbleJob a, const NibbleJob b, int blocks_a) {
+  const bool first = (int)blockIdx.x < blocks_a;
+  const uint32_t* __restrict__ planes = first ? a.planes : b.planes;
+  uint8_t* __restrict__ out = first ? a.out : b.out;
+  const long long total = first ? a.total : b.total;
+  const int bits = first ? a.bits : b.bits, is_signed = first ? a.is_signed : b.is_signed;
+  const long long nblk = first ? blocks_a : (long long)gridDim.x - blocks_a;
+  const long long blk = first ? blockIdx.x : (long long)blockIdx.x - blocks_a;
+  grid_dependency_wait();   // launched as a programmatic dependent: nothing global is touched before this
   // four words per thread and trip, their loads issued together
   constexpr int U = 4;
-  const long long step = (long long)gridDim.x * blockDim.x;
-  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += U * step) {
+  const long long step = nblk * blockDim.x;
+  for (long long i0 = blk * blockDim.x + threadIdx.x; i0 < total; i0 += U * step) {
     uint32_t w0[U], w1[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
@@ -818,16 +832,34 @@ apnn_status tc5_gemm_i8_pair(cudaStream_t s, const uint8_t* A8, const uint8_t* B
   return APNN_OK;
 }
 
-apnn_status tc5_expand_fp4(cudaStream_t s, const uint32_t* planes, uint8_t* out, long long rows, int K, int bits,
-                           bool is_signed) {
-  const long long total = rows * (K / 32);
-  long long blocks = (total + 4 * 256 - 1) / (4 * 256), cap = (long long)device_sm_count() * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-  expand_nibbles_kernel<<<(int)blocks, 256, 0, s>>>(planes, out, total, bits, is_signed ? 1 : 0);
-  cudaError_t e = cudaGetLastError();
+// One launch for one operand (rows_b == 0) or both operands of a contraction.  rows x K only counts words here: planes
+// and nibble rows are both linear in the 32-k words.
+apnn_status tc5_expand2_fp4(cudaStream_t s, const uint32_t* pa, uint8_t* oa, long long rows_a, int bits_a, bool signed_a,
+                            const uint32_t* pb, uint8_t* ob, long long rows_b, int bits_b, bool signed_b, int K) {
+  const long long cap = (long long)device_sm_count() * 8;
+  auto blocks_for = [cap](long long total) {
+    long long b = (total + 4 * 256 - 1) / (4 * 256);
+    return (int)(b > cap ? cap : b);
+  };
+  const NibbleJob a = {pa, oa, rows_a * (K / 32), bits_a, signed_a ? 1 : 0};
+  const NibbleJob b = {pb, ob, rows_b * (K / 32), bits_b, signed_b ? 1 : 0};
+  const int ba = blocks_for(a.total), bb = blocks_for(b.total);
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)(ba + bb), 1, 1);
+  cfg.blockDim = dim3(256, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = (unsigned)pdl_attribute(attr);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, expand_nibbles_kernel, a, b, ba);
   if (e != cudaSuccess) return cuda_fail(e, "expand_nibbles launch");
   return APNN_OK;
+}
+
+apnn_status tc5_expand_fp4(cudaStream_t s, const uint32_t* planes, uint8_t* out, long long rows, int K, int bits,
+                           bool is_signed) {
+  return tc5_expand2_fp4(s, planes, out, rows, bits, is_signed, nullptr, nullptr, 0, 1, false, K);
 }
 
 // D = A4 * B4^T over e2m1 nibble rows (K/2 bytes per row, K a multiple of 256), int32 or packed outputs.

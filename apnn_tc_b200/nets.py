@@ -457,13 +457,6 @@ class Network:
         for ls in spec.layers:
             users = [c.name for c in spec.layers if self.src_of[c.name] == ls.name]
             if use_tcgen05 and ls.quantise and users and self.tc5_ok[ls.name] and all(self.tc5_ok[u] for u in users):
-                sh = self.params[ls.name].shape
-                if ls.kind == "conv":
-                    hh = halo[ls.name]
-                    shape = (B, sh["Ho"] + 2 * hh, sh["Wo"] + 2 * hh, sh["coutp"])
-                else:
-                    shape = (B, sh["coutp"])
-                self.out[ls.name] = torch.zeros(shape, dtype=torch.uint8, device=self.device)
                 self.i8_out[ls.name] = True
         # pooled stride-1 layers whose output leaves as int8 rows run the (faster) flat convolution
         # unpooled into a scratch map and pool the level bytes afterwards: with ascending thresholds
@@ -478,6 +471,13 @@ class Network:
                 self.split_pool[ls.name] = True
                 pool_bytes = max(pool_bytes, B * 2 * sh["Ho"] * 2 * sh["Wo"] * sh["coutp"])
         self.unpooled = torch.empty(max(pool_bytes, 16), dtype=torch.uint8, device=self.device)
+        self._plan_fp4()
+        for ls in spec.layers:
+            if self.i8_out.get(ls.name, False):
+                sh, hh = self.params[ls.name].shape, halo[ls.name]
+                pixels = (sh["Ho"] + 2 * hh, sh["Wo"] + 2 * hh) if ls.kind == "conv" else ()
+                width = sh["coutp"] // 2 if self.fp4_out.get(ls.name, False) else sh["coutp"]
+                self.out[ls.name] = torch.zeros((B,) + pixels + (width,), dtype=torch.uint8, device=self.device)
         if self.first_im2col is None:
             self.image_planes = torch.zeros((a, B, self.hw + 2 * h0, self.hw + 2 * h0, cp // 32), dtype=torch.int32,
                                             device=self.device)
@@ -490,11 +490,54 @@ class Network:
         self.launches_per_forward = 0
         torch.cuda.synchronize(self.device)
 
+    def _fp4_candidate(self, ls: LayerSpec) -> bool:
+        """Hidden stride-1 convolutions the e2m1 kernel takes and runs faster than the int8 one: weights and activations of
+        at most two bits, 128-channel inputs, and at least one whole 256-channel tile of outputs (128 x 28x28, 128 -> 128
+        channels fills half a tile: 25 us against 20 on int8; 128 -> 256 and wider: 0.55 - 0.65 of the int8 time).  Layers
+        with residuals stay on int8, whose epilogue fetches them ahead (1024 x 14x14, 256 channels: 115 us against 123)."""
+        if ls.residual_from or ls.save_residual:
+            return False
+        if ls.kind != "conv" or not self.i8_out.get(self.src_of[ls.name], False) or ls.stride != 1 or ls.R not in (1, 3):
+            return False
+        sh = self.params[ls.name].shape
+        ring = self.halo[self.src_of[ls.name]]
+        return (self.spec.a_bit <= 2 and self.spec.w_bit == 1 and sh["cinp"] % 128 == 0 and sh["coutp"] >= 256
+                and 9 * ls.R * ls.R * sh["cinp"] < 2 ** 24 and (ls.R == 1 or sh["W"] + 2 * ring <= 100)
+                and (ls.pool != 2 or self.split_pool.get(ls.name, False)))
+
+    def _plan_fp4(self) -> None:
+        """Which layers run on e2m1 operands (``fp4``) and which outputs are stored as nibble rows (``fp4_out``: every
+        consumer takes them).  APNN_FP4=0 in the environment keeps everything on int8."""
+        self.fp4: Dict[str, bool] = {}
+        self.fp4_out: Dict[str, bool] = {}
+        self.w4: Dict[str, torch.Tensor] = {}
+        if os.environ.get("APNN_FP4", "1") == "0":
+            return
+        users = {ls.name: [c for c in self.spec.layers if self.src_of[c.name] == ls.name] for ls in self.spec.layers}
+        for ls in self.spec.layers:
+            if ls.kind == "conv" and self.i8_out.get(ls.name, False) and all(self._fp4_candidate(u) for u in users[ls.name]):
+                self.fp4_out[ls.name] = True
+                for u in users[ls.name]:
+                    wp = self.w_planes[u.name]
+                    w4 = torch.empty(wp.numel() * 16, dtype=torch.uint8, device=self.device)
+                    _cabi.check(self.L.apnn_expand_planes_fp4(_stream_ptr(), wp.data_ptr(), w4.data_ptr(), wp.numel() // 8, 256,
+                                                              1, 1), "expand weights")
+                    self.w4[u.name] = w4
+                    self.w8.pop(u.name, None)
+                    self.fp4[u.name] = True
+
     # -- one layer -------------------------------------------------------------------
     def levels_of(self, name: str) -> torch.Tensor:
         """Quantised output of a layer as levels [B, (H, W,) C] without its ring, whichever form it is stored in."""
         t, h = self.out[name], self.halo.get(name, 0)
-        if self.i8_out.get(name, False):
+        if self.fp4_out.get(name, False):
+            # nibble 2i + (q >> 2) of word q & 3 of a 32-channel group is byte 4q + i of the int8 form
+            e = torch.arange(32, device=t.device)
+            bit = 31 - e
+            code = (torch.stack((t & 15, t >> 4), dim=-1)).reshape(t.shape[:-1] + (t.shape[-1] // 16, 32))
+            code = code[..., 8 * (bit & 3) + (bit >> 2)].reshape(t.shape[:-1] + (t.shape[-1] * 2,))
+            g = (code >> 1) + (code & 1)      # codes 0, 2, 4, 5
+        elif self.i8_out.get(name, False):
             e = torch.arange(32, device=t.device)
             pos = 4 * ((31 - e) & 7) + ((31 - e) >> 3)      # byte of element e inside a group of 32 channels
             g = t.reshape(t.shape[:-1] + (t.shape[-1] // 32, 32))[..., pos].reshape(t.shape)
@@ -524,7 +567,8 @@ class Network:
                              pool="max" if (ls.pool == 2 and not split) else "none",
                              out_halo=self.halo[ls.name] if (conv and not split) else 0,
                              in_halo=self.halo[self.src_of[ls.name]] if conv else 0, thresholds=self.thr[ls.name],
-                             residual_in=res_in, residual_out=res_out, out_i8=self.i8_out.get(ls.name, False),
+                             residual_in=res_in, residual_out=res_out,
+                             out_i8=(_cabi.ROWS_FP4 if self.fp4_out.get(ls.name, False) else self.i8_out.get(ls.name, False)),
                              residual_i16=r16)
 
     def _run_conv(self, ls: LayerSpec) -> int:
@@ -536,9 +580,14 @@ class Network:
         s = _stream_ptr()
         if self.split_pool.get(ls.name, False):
             final, out = out, self.unpooled
+            # the scratch map holds nibbles where an e2m1 layer feeds another one, else bytes
+            nib_in = self.fp4.get(ls.name, False) and self.fp4_out.get(ls.name, False)
+            epi.out_i8 = _cabi.ROWS_FP4 if nib_in else _cabi.ROWS_I8
             n = self._launch_conv(ls, sh, X, a, B, epi, out, s)
-            _cabi.check(self.L.apnn_maxpool2x2_i8(s, out.data_ptr(), final.data_ptr(), B, 2 * sh["Ho"], 2 * sh["Wo"],
-                                                  sh["coutp"], 0, self.halo[ls.name]), "apnn_maxpool2x2_i8 " + ls.name)
+            _cabi.check(self.L.apnn_maxpool2x2_rows(s, out.data_ptr(), final.data_ptr(), B, 2 * sh["Ho"], 2 * sh["Wo"],
+                                                    sh["coutp"], 0, self.halo[ls.name], int(epi.out_i8),
+                                                    _cabi.ROWS_FP4 if self.fp4_out.get(ls.name, False) else _cabi.ROWS_I8),
+                        "apnn_maxpool2x2_rows " + ls.name)
             return n + 1
         return self._launch_conv(ls, sh, X, a, B, epi, out, s)
 
@@ -559,15 +608,21 @@ class Network:
                                               Hc, Wc, kp, sh["coutp"], 1, 1, signs, ctypes.byref(epi), self.flag.data_ptr()),
                         "apnn_conv2d_i8 " + ls.name)
             return 1
+        if self.fp4.get(ls.name, False):
+            _cabi.check(self.L.apnn_conv2d_fp4(s, self.w4[ls.name].data_ptr(), X.data_ptr(), out.data_ptr(), B, sh["H"],
+                                               sh["W"], sh["cinp"], sh["coutp"], ls.R, ctypes.byref(epi),
+                                               self.flag.data_ptr()), "apnn_conv2d_fp4 " + ls.name)
+            return 1
         if self.tc5_ok[ls.name]:
             n, x8 = 1, X
             if not self.i8_out.get(self.src_of[ls.name], False):
                 rows = X.shape[1] * X.shape[2] * X.shape[3]
                 _cabi.check(self.L.apnn_expand_planes(s, X.data_ptr(), self.x8.data_ptr(), rows, sh["cinp"], a, 0), "expand")
                 n, x8 = 2, self.x8
-            _cabi.check(self.L.apnn_conv2d_i8(s, self.w8[ls.name].data_ptr(), x8.data_ptr(), out.data_ptr(), B,
-                                              sh["H"], sh["W"], sh["cinp"], sh["coutp"], ls.R, ls.stride, 1,
-                                              ctypes.byref(epi), self.flag.data_ptr()), "apnn_conv2d_i8 " + ls.name)
+            conv = self.L.apnn_conv2d_i8_to_fp4 if epi.out_i8 == _cabi.ROWS_FP4 else self.L.apnn_conv2d_i8
+            _cabi.check(conv(s, self.w8[ls.name].data_ptr(), x8.data_ptr(), out.data_ptr(), B,
+                             sh["H"], sh["W"], sh["cinp"], sh["coutp"], ls.R, ls.stride, 1,
+                             ctypes.byref(epi), self.flag.data_ptr()), "apnn_conv2d_i8 " + ls.name)
             return n
         epi.signed_operand = _cabi.SIGN_W
         _cabi.check(self.L.apnn_conv2d_ex(s, _cabi.ALGO_IMMA, 1, a, self.w_planes[ls.name].data_ptr(), X.data_ptr(),

@@ -65,7 +65,7 @@ def make_epilogue(out_mode: str = "int32", out_bits: int = 0, signed: str = "non
     e.residual_in = residual_in.data_ptr() if residual_in is not None else None
     e.residual_out = residual_out.data_ptr() if residual_out is not None else None
     e.residual_i16 = int(residual_i16)   # bit 0: residual_in is int16, bit 1: residual_out is int16 (gemm_i8 / conv2d_i8)
-    e.out_i8 = 1 if out_i8 else 0   # one byte per output element instead of packed planes (gemm_i8 / conv2d_i8)
+    e.out_i8 = int(out_i8)   # 1: one byte per output element instead of packed planes (gemm_i8 / conv2d_i8); 2: one e2m1 nibble
     if peer_out:
         if len(peer_out) > 7:
             raise ValueError("at most 7 peer destinations")

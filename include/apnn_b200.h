@@ -260,6 +260,22 @@ apnn_status apnn_conv2d_i8(void *stream, const void *W8, const void *X8, void *O
                            int CIN, int COUT, int R, int stride, int w_signed,
                            const apnn_epilogue *epi, int *status_flag);
 
+/* The stride-1 convolution of apnn_conv2d_i8 on operands of at most two bits in e2m1 nibbles (see
+ * apnn_expand_planes_fp4; filter rows W4[COUT][R*R*CIN/2], activations X4[B][H+2h][W+2h][CIN/2]) at
+ * twice the int8 tensor rate, bit for bit the same results.  R is 1 or 3, CIN % 128 == 0, the sums
+ * stay below 2^24 (9*R*R*CIN < 2^24), no pooling, no APNN_OUT_FLOAT, and the image is at most about
+ * 100 pixels wide for R = 3 (the rows the taps of a tile reach must fit one 256-row box), else
+ * APNN_ERR_UNSUPPORTED.  epi->out_i8 = 1 writes int8 rows, APNN_ROWS_FP4 nibble rows (out_bits <= 2):
+ * the operand of the next such layer.  No reference counterpart. */
+#define APNN_ROWS_FP4 2
+apnn_status apnn_conv2d_fp4(void *stream, const void *W4, const void *X4, void *Out, int B, int H, int W,
+                            int CIN, int COUT, int R, const apnn_epilogue *epi, int *status_flag);
+
+/* apnn_conv2d_i8 (int8 operands) whose quantised output leaves as e2m1 nibble rows: epi->out_i8 = APNN_ROWS_FP4. */
+apnn_status apnn_conv2d_i8_to_fp4(void *stream, const void *W8, const void *X8, void *Out, int B, int H, int W,
+                                  int CIN, int COUT, int R, int stride, int w_signed,
+                                  const apnn_epilogue *epi, int *status_flag);
+
 /* The quantising part of the epilogue on its own: int32 values[rows][N] -> levels (out_mode
  * APNN_OUT_LOWBITS or APNN_OUT_THRESHOLDS with epi->thresholds [N][2^out_bits - 1]) -> packed
  * planes [out_bits][rows][N/32], or int8 rows [rows][N] when epi->out_i8 is set; with APNN_OUT_FLOAT
@@ -280,6 +296,12 @@ apnn_status apnn_requantize_i32(void *stream, const int32_t *values, void *out, 
  * binarised outputs = maximum of 1-bit levels). */
 apnn_status apnn_maxpool2x2_i8(void *stream, const void *in_i8, void *out_i8, int B, int H, int W, int C,
                                int in_halo, int out_halo);
+
+/* The same with a form for each side: in_form / out_form 1 = int8 rows, APNN_ROWS_FP4 = e2m1 nibble rows (levels
+ * 0..3; their codes are ordered like the levels, so the maximum of the codes is the code of the maximum).
+ * C % 32 == 0; an int8 output of a nibble input is not taken. */
+apnn_status apnn_maxpool2x2_rows(void *stream, const void *in, void *out, int B, int H, int W, int C,
+                                 int in_halo, int out_halo, int in_form, int out_form);
 
 /* ---- packers -------------------------------------------------------------------
  * apnn_bit_compress replaces Bit_compression (NN/kernel.cuh:46-77): one uint32 level per
