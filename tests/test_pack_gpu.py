@@ -185,3 +185,25 @@ def test_quantize_blocks_i8_refuses_what_it_does_not_cover(cuda_device):
     assert L.apnn_quantize_blocks_i8(s, x.data_ptr(), out.data_ptr(), 1, 8, 8, 3, 2, 8, 1, 64) == 2    # stride * C = 6: no whole quads
     assert L.apnn_quantize_blocks_i8(s, x.data_ptr(), out.data_ptr(), 1, 8, 8, 3, 4, 8, 1, 32) == 2    # 48 level bytes > cpad
     assert L.apnn_quantize_blocks_i8(s, x.data_ptr(), out.data_ptr(), 1, 7, 8, 3, 4, 8, 1, 64) == 2    # H not a multiple of stride
+
+
+@pytest.mark.parametrize("rows,C,bits", [(1, 33, 1), (3, 129, 7), (9, 131, 3), (17, 256, 2), (2, 1023, 5), (700, 384, 2), (40000, 128, 1),
+                                         (1, 9, 2), (5, 12, 3), (37, 32, 8), (100003, 30, 2), (90001, 24, 4)])
+@pytest.mark.parametrize("source", ["levels", "float"])
+def test_pack_groups_of_a_trip(cuda_device, rows, C, bits, source):
+    """Trips of eight 128-channel groups: partial last trips, rows that end inside a trip, ragged rows, several trips."""
+    import apnn_tc_b200 as ap
+    rng = np.random.default_rng(rows * C)
+    if source == "levels":
+        lv = rng.integers(0, 1 << 32, size=(rows, C), dtype=np.uint32)      # only the low bits count
+        got = to_host(ap.Bit_compression(to_dev(lv), bits))
+        assert np.array_equal(got, oracle.bit_compress(lv & ((1 << bits) - 1), bits))
+        return
+    x = rng.uniform(-12, 12, size=(rows, C)).astype(np.float32)
+    step = 20.0 / (1 << bits)
+    edges = (-10 + step * (np.arange(1 << bits) + 0.5)).astype(np.float32)
+    probe = np.concatenate([edges, np.nextafter(edges, np.float32(-20)), np.nextafter(edges, np.float32(20)),
+                            np.array([-10, 10, -np.inf, np.inf, -0.0], np.float32)])
+    x.reshape(-1)[: min(probe.size, x.size)] = probe[: x.size]
+    got = to_host(ap.images_quantization(torch.from_numpy(x).cuda(), bits))
+    assert np.array_equal(got, oracle.bit_compress(oracle.quantize(x, bits), bits))
