@@ -357,6 +357,22 @@ apnn_status apnn_conv2d_fp4(void* stream, const void* W4, const void* X4, void* 
                       R, epi, status_flag);
 }
 
+apnn_status apnn_linear_fp4(void* stream, const void* X4, const void* W4, void* Out, int M, int N, int K,
+                            const apnn_epilogue* epi, int* status_flag) {
+  if (!X4 || !W4 || !Out || !status_flag || M <= 0 || N <= 0 || K <= 0) return APNN_ERR_INVALID_ARG;
+  if (K % 128 != 0 || !aligned16(X4) || !aligned16(W4) || !aligned16(Out)) return APNN_ERR_ALIGNMENT;
+  if (epi) {
+    if (epi->signed_operand != APNN_SIGN_NONE) return APNN_ERR_INVALID_ARG;
+    apnn_status st = check_epilogue(epi, N, false, 1, 1, true, true);
+    if (st == APNN_OK && epi->out_i8 == 1 && !aligned32(Out)) st = APNN_ERR_ALIGNMENT;
+    if (st != APNN_OK) return st;
+    if (epi->n_peer_out != 0) return APNN_ERR_UNSUPPORTED;
+  }
+  if (tc5_gemm_fp4_flat_clocks(M, N, K) == 0) return APNN_ERR_UNSUPPORTED;
+  return tc5_gemm_fp4_flat(reinterpret_cast<cudaStream_t>(stream), (const uint8_t*)X4, (const uint8_t*)W4, Out, M, N, K, epi,
+                           status_flag);
+}
+
 apnn_status apnn_conv2d(void* stream, int wbits, int xbits, const void* Wt, const void* X, void* Out, int B, int H,
                         int Wd, int CIN, int COUT, int R, int stride, const apnn_epilogue* epi) {
   return apnn_conv2d_ex(stream, APNN_ALGO_IMMA, wbits, xbits, Wt, X, Out, B, H, Wd, CIN, COUT, R, stride, epi, nullptr,

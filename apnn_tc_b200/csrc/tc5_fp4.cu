@@ -26,8 +26,10 @@
 // tmem_empty in the leader (every epilogue warp of both CTAs).  All waits are time-bounded.  The loads carry no cluster multicast.
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 
 #include "api_internal.h"
+#include "fp4_epilogue.cuh"
 #include "tc5_common.cuh"
 #include "tc5_gemm.h"
 
@@ -36,8 +38,8 @@ namespace apnn {
 namespace {
 
 using namespace tc5;
+using namespace fp4;
 
-constexpr int HALF = 128;               // channels of one CTA
 constexpr int TILE_CH = 2 * HALF;       // channels of a pair's tile
 constexpr int MAX_NP = 224;             // pixels of a tile: a multiple of 32
 constexpr uint32_t SF_COL = 2 * MAX_NP; // 32 TMEM columns of scale factors, every byte ue8m0 1.0 (0x7F)
@@ -51,29 +53,6 @@ constexpr int MAX_NA = 8, MAX_NB = 8;   // ring depths
 constexpr int BAR_BYTES = 512;
 constexpr int ROWS_BYTES = epi_warps(0, 64) * 64 * 4;   // per epilogue warp: the output rows of a chunk's 32 pixels
 constexpr int SMEM_LIMIT = 232448;
-
-struct Fp4Params {
-  void* out;
-  const int32_t* thresholds;
-  const int32_t* residual_in;
-  int32_t* residual_out;
-  int N, cblocks, cin_bytes;
-  int np, tiles_m, tiles_n;
-  int out_mode, out_bits;
-  int rows_out;                // 0: packed planes, 1: int8 rows, 2: e2m1 nibble rows
-  int res16_in, res16_out;
-  long long out_plane_words;
-  int wp, hpwp, in_off;
-  int Bn, Ho, Wo, out_halo;
-  unsigned long long magic_hpwp, magic_wp;   // n / d == (n * magic) >> shift for 0 <= n < 2^31
-  int shift_hpwp, shift_wp;
-  uint32_t a_bytes;            // bytes of one CTA's pixel box
-  uint32_t a_buf;              // its buffer, a multiple of 1024
-  int na, nb;                  // ring depths: pixel boxes, filter stages
-  int w_resident;              // one channel tile and one K block: the R filter stages are loaded once and stay
-  uint32_t idesc;
-  int* error_flag;
-};
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -102,10 +81,11 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
       "[%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar_cluster)
       : "memory");
 }
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+// pair_mask: the two CTAs of this pair as bits of the cluster rank
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint16_t pair_mask) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"((uint16_t)3)
+      "h"(pair_mask)
       : "memory");
 }
 __device__ __forceinline__ void tc_mma_mxf4_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -117,121 +97,15 @@ __device__ __forceinline__ void tc_mma_mxf4_pair(uint32_t d_tmem, uint64_t adesc
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(sf_tmem), "r"(sf_tmem + 16u), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tmem_fill8(uint32_t taddr, uint32_t v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(v) : "memory");
-}
 
-// 32 x 32 bit transposition over the warp: bit b of lane a <-> bit a of lane b.
-__device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane) {
-#pragma unroll
-  for (int s = 16; s >= 1; s >>= 1) {
-    const uint32_t low = s == 16 ? 0x0000FFFFu : s == 8 ? 0x00FF00FFu : s == 4 ? 0x0F0F0F0Fu : s == 2 ? 0x33333333u : 0x55555555u;
-    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, s);
-    const bool up = (lane & s) != 0;
-    const uint32_t rot = __funnelshift_l(y, y, up ? 32 - s : s);
-    const uint32_t keep = up ? ~low : low;
-    x = (x & keep) | (rot & ~keep);
-  }
-  return x;
-}
-
-// Bit j of each result: v[j] (a float integer) lies below the threshold whose negation nt holds (twice).  The sign bit of
-// v + nt is that bit: one packed addition per two values, one PRMT that replicates two sign bits into bytes and one masked
-// OR -- compare-and-set through predicates ran at 6 clk per instruction with the two warps a scheduler has here (13-cycle
-// predicate latency): 128 x 56x56, 256 -> 256 channels went from 127 to 109 us with this form and the early reload below.
-__device__ __forceinline__ uint32_t below_bits(const uint32_t (&v)[32], unsigned long long nt) {
-  uint32_t w[2] = {0u, 0u};
-#pragma unroll
-  for (int h = 0; h < 2; h++) {   // elements 16h + i and 16h + 8 + i share a PRMT
-    uint32_t e[16];
-#pragma unroll
-    for (int i = 0; i < 16; i += 2) {
-      unsigned long long x, d;
-      asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(v[16 * h + i]), "r"(v[16 * h + i + 1]));
-      asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(nt));
-      asm("mov.b64 {%0, %1}, %2;" : "=r"(e[i]), "=r"(e[i + 1]) : "l"(d));
-    }
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      uint32_t s;
-      asm("prmt.b32 %0, %1, %2, 0xFBFB;" : "=r"(s) : "r"(e[i]), "r"(e[i + 8]));
-      w[h] |= s & (0x0101u << (16 * h + i));
-    }
-  }
-  return w[0] | w[1];
-}
-// -t in both halves; a zero threshold stays +0, so that +0 and -0 sums both land on its upper side
-__device__ __forceinline__ unsigned long long negated2(float t) {
-  const uint32_t u = t == 0.0f ? 0u : __float_as_uint(-t);
-  return ((unsigned long long)u << 32) | u;
-}
-
-// Level words of one pixel (bit 31 - c = channel c of the 32-channel group, one word per bit) -> the pixel's 16 bytes of
-// e2m1 nibbles, in expand_nibbles_kernel's order: nibble i of word q holds the element at bit 4i + q.
-__device__ __forceinline__ uint4 nibbles_of(uint32_t p0, uint32_t p1) {
-  uint32_t o[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const uint32_t t0 = (p0 >> q) & 0x11111111u, t1 = (p1 >> q) & 0x11111111u;
-    o[q] = (t1 << 2) | ((t0 & ~t1) << 1) | (t0 & t1);
-  }
-  return make_uint4(o[0], o[1], o[2], o[3]);
-}
-__device__ __forceinline__ void store_32(uint8_t* dst, const uint32_t (&r)[8]) {
-  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),
-               "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-
-// Accesses of one pixel's row, left out when row < 0: predicated instructions (as `if`s they became a branch each, and the
-// int32 epilogue of 128 x 56x56, 256 channels took 160 us instead of 119).
-__device__ __forceinline__ void st_row32(int32_t* base, int row, int pitch, uint32_t x) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p st.global.b32 [%0], %1;\n\t}" ::"l"(base + (long long)row * pitch), "r"(x),
-               "r"(row)
-               : "memory");
-}
-__device__ __forceinline__ void st_row16(int16_t* base, int row, int pitch, uint32_t x) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\t@p st.global.b16 [%0], %1;\n\t}" ::"l"(base + (long long)row * pitch),
-               "h"((uint16_t)x), "r"(row)
-               : "memory");
-}
-__device__ __forceinline__ int ld_row32(const int32_t* base, int row, int pitch) {
-  int x;
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.nc.b32 %0, [%1];\n\t}"
-               : "=r"(x)
-               : "l"(base + (long long)row * pitch), "r"(row));
-  return x;
-}
-__device__ __forceinline__ int ld_row16(const int16_t* base, int row, int pitch) {
-  int x;
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ge.s32 p, %2, 0;\n\tmov.b32 %0, 0;\n\t@p ld.global.nc.s16 %0, [%1];\n\t}"
-               : "=r"(x)
-               : "l"(base + (long long)row * pitch), "r"(row));
-  return x;
-}
-
-struct PixelRow {
-  int row;     // output row, ring included; -1 when the position is not an output pixel
-  int dense;   // output row without the ring (index of the residual tensors)
-};
-__device__ __forceinline__ PixelRow pixel_row(const Fp4Params& p, long long pos) {
-  PixelRow r = {-1, -1};
-  if (pos >= 0x7fffffffLL) return r;
-  const uint32_t n = (uint32_t)pos;
-  const int b = (int)(((unsigned long long)n * p.magic_hpwp) >> p.shift_hpwp);
-  const uint32_t rem = n - (uint32_t)b * (uint32_t)p.hpwp;
-  const int ho = (int)(((unsigned long long)rem * p.magic_wp) >> p.shift_wp);
-  const int wo = (int)(rem - (uint32_t)ho * (uint32_t)p.wp);
-  if (b < p.Bn && ho < p.Ho && wo < p.Wo) {
-    r.row = (b * (p.Ho + 2 * p.out_halo) + ho + p.out_halo) * (p.Wo + 2 * p.out_halo) + wo + p.out_halo;
-    r.dense = (b * p.Ho + ho) * p.Wo + wo;
-  }
-  return r;
-}
-
-// EPI 1: thresholds of at most two bits -> planes, int8 rows or nibble rows, no residuals; 2: the same with int16 residuals
-// in and / or out, added as floats (the host checks that the sums stay below 2^24); 0: everything else.
-template <int RR, int BKB, int EPI>
+// EPI: the epilogue family of finish_chunk.
+//
+// SPLIT: a problem with fewer tiles than SM pairs and a long K (the fully connected layers) is launched as clusters of
+// p.splits pairs that share one tile.  Each pair sums its part of the K blocks in its own TMEM; then 32-pixel chunk c goes
+// to pair c % splits: the others store their partial sums of it into that pair's idle operand ring (distributed shared
+// memory, one 16 KiB slot per source and chunk), and after a cluster barrier the owner adds the slots to its own sums --
+// integers below 2^24, so the order does not matter -- and runs the ordinary epilogue on the chunk.
+template <int RR, int BKB, int EPI, bool SPLIT>
 __global__ void __launch_bounds__(threads_of(EPI, BKB), 1)
 tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const Fp4Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -240,7 +114,7 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   constexpr uint32_t TAP_BYTES = HALF * BKB;
   constexpr uint32_t STAGE_BYTES = RR * TAP_BYTES;
   const uint32_t wring = base + (uint32_t)p.na * p.a_buf;
-  const uint32_t bars = wring + (uint32_t)p.nb * STAGE_BYTES;
+  const uint32_t bars = base + p.ring_bytes;
   auto xfull_bar = [&](int i) { return bars + 8u * i; };
   auto xempty_bar = [&](int i) { return bars + 8u * (MAX_NA + i); };
   auto wfull_bar = [&](int s) { return bars + 8u * (2 * MAX_NA + s); };
@@ -253,9 +127,14 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();   // 0 = leader
-  const int pair = blockIdx.x >> 1;
-  const int num_pairs = gridDim.x >> 1;
+  const uint32_t crank = cluster_ctarank();
+  const uint32_t rank = crank & 1u;          // 0 = the pair's leader
+  const uint32_t leader = SPLIT ? crank & ~1u : 0u;
+  const int split = SPLIT ? (int)(crank >> 1) : 0;
+  const int pair = SPLIT ? (int)blockIdx.x / (2 * p.splits) : (int)blockIdx.x >> 1;   // the pair's, or cluster's, first tile
+  const int num_pairs = SPLIT ? (int)gridDim.x / (2 * p.splits) : (int)gridDim.x >> 1;
+  const int cb0 = SPLIT ? split * p.cblocks / p.splits : 0;
+  const int cb1 = SPLIT ? (split + 1) * p.cblocks / p.splits : p.cblocks;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.na; i++) {
@@ -306,17 +185,17 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
         const int q0 = tm * p.np + (int)rank * (p.np >> 1) + p.in_off * p.wp + p.in_off;
         const int wrow = tn * TILE_CH + (int)rank * HALF;
-        for (int cb = 0; cb < p.cblocks && ok; cb++) {
+        for (int cb = cb0; cb < cb1 && ok; cb++) {
           if (!mbar_wait(xempty_bar(ia), pha ^ 1u)) { ok = false; break; }
           if (rank == 0) mbar_expect_tx(xfull_bar(ia), 2 * p.a_bytes);   // both CTAs' bytes
-          tma_load_2d_pair(base + (uint32_t)ia * p.a_buf, &map_x, cb * BKB, q0, map_to_cta(xfull_bar(ia), 0));
+          tma_load_2d_pair(base + (uint32_t)ia * p.a_buf, &map_x, cb * BKB, q0, map_to_cta(xfull_bar(ia), leader));
           if (++ia == p.na) { ia = 0; pha ^= 1u; }
           int kcol = cb * BKB;
           if (p.w_resident && tile != pair) continue;
           for (int ti = 0; ti < RR; ti++) {
             if (!mbar_wait(wempty_bar(sb), phb ^ 1u)) { ok = false; break; }
             if (rank == 0) mbar_expect_tx(wfull_bar(sb), 2 * STAGE_BYTES);
-            const uint32_t full = map_to_cta(wfull_bar(sb), 0);
+            const uint32_t full = map_to_cta(wfull_bar(sb), leader);
 #pragma unroll
             for (int tj = 0; tj < RR; tj++, kcol += p.cin_bytes)
               tma_load_2d_pair(wring + (uint32_t)sb * STAGE_BYTES + tj * TAP_BYTES, &map_w, kcol, wrow, full);
@@ -326,6 +205,11 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       }
       if (!ok) atomicExch(p.error_flag, 1);
     }
+    if constexpr (SPLIT) {   // the two cluster barriers of the exchange (every thread takes part)
+      __syncwarp();
+      cluster_sync_all();
+      cluster_sync_all();
+    }
   } else if (warp == 1) {
     // ---------------- MMA issuer (leader CTA only) ----------------
     if (lane == 0 && rank == 0) {
@@ -334,6 +218,7 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
       uint32_t tl = 0;
       bool ok = true;
       const uint32_t sf = tmem_base + SF_COL;
+      const uint16_t pair_mask = (uint16_t)(3u << leader);
       const uint32_t row_step = (uint32_t)p.wp * (BKB / 16);
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, tl++) {
         const uint32_t acc = tl & 1u;
@@ -342,7 +227,7 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * MAX_NP;
         uint32_t enable = 0;
-        for (int cb = 0; cb < p.cblocks && ok; cb++) {
+        for (int cb = cb0; cb < cb1 && ok; cb++) {
           if (!mbar_wait(xfull_bar(ia), pha)) { ok = false; break; }
           tc_fence_after();
           const uint64_t x0 = make_smem_desc_k<BKB>(base + (uint32_t)ia * p.a_buf);
@@ -364,15 +249,20 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
                 enable = 1u;
               }
             }
-            if (!p.w_resident) tc_commit_pair(wempty_bar(sb));   // frees the filter stage in both CTAs
+            if (!p.w_resident) tc_commit_pair(wempty_bar(sb), pair_mask);   // frees the filter stage in both CTAs
             if (++sb == p.nb) { sb = 0; phb ^= 1u; }
           }
-          if (ok) tc_commit_pair(xempty_bar(ia));   // frees the pixel box in both CTAs
+          if (ok) tc_commit_pair(xempty_bar(ia), pair_mask);   // frees the pixel box in both CTAs
           if (++ia == p.na) { ia = 0; pha ^= 1u; }
         }
-        if (ok) tc_commit_pair(tfull_bar(acc));   // accumulators complete in both CTAs
+        if (ok) tc_commit_pair(tfull_bar(acc), pair_mask);   // accumulators complete in both CTAs
       }
       if (!ok) atomicExch(p.error_flag, 2);
+    }
+    if constexpr (SPLIT) {
+      __syncwarp();
+      cluster_sync_all();
+      cluster_sync_all();
     }
   } else {
     // ---------------- epilogue warps of both CTAs ----------------
@@ -383,215 +273,73 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     uint32_t tl = 0;
     bool ok = true;
     int thr_tn = -1;
-    // the float comparison is exact: |value| < 2^24 is a float, and rounding a larger threshold keeps its side.  A missing
-    // threshold is +inf (its negation -inf).
-    unsigned long long nt1 = 0ull, nt2 = 0xff800000ff800000ull, nt3 = nt2;
+    ChannelThresholds thr;
     int* rows_s = reinterpret_cast<int*>(smem_raw + (bars + BAR_BYTES - raw)) + (warp - 2) * 64;   // rows, then dense rows
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, tl++) {
       const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
       const int ch0 = tn * TILE_CH + (int)rank * HALF + quarter * 32;   // this warp's 32 channels
-      const int ch = ch0 + lane;
       if (EPI != 0 && tn != thr_tn) {
-        if (ch < p.N) {
-          const int32_t* T = p.thresholds + (long long)ch * nl;
-          nt1 = negated2((float)__ldg(T));
-          if (nl > 1) {
-            nt2 = negated2((float)__ldg(T + 1));
-            nt3 = negated2((float)__ldg(T + 2));
-          }
-        }
+        if (ch0 + lane < p.N) thr.load(p.thresholds + (long long)(ch0 + lane) * nl, nl);
         thr_tn = tn;
       }
       const uint32_t acc = tl & 1u;
       const uint32_t aph = (tl >> 1) & 1u;
-      if (!mbar_wait(tfull_bar(acc), aph)) { ok = false; break; }
+      const bool acc_ok = mbar_wait(tfull_bar(acc), aph);
+      if (!acc_ok) ok = false;
+      if (!SPLIT && !acc_ok) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * MAX_NP;
+      // 16-byte groups of 4 pixels, group g of channel row r of slot n at ((8 n + g) * 128 + r) * 16
+      const uint32_t slot_row = base + (uint32_t)(quarter * 32 + lane) * 16u;
+      if constexpr (SPLIT) {
+        __syncwarp();
+        cluster_sync_all();   // every accumulator of the cluster is complete, every operand ring idle
+        if (acc_ok) {
+#pragma unroll 1
+          for (int c = part; c * 32 < p.np; c += PARTS) {
+            const int owner = c % p.splits;
+            if (owner == split) continue;
+            uint32_t x[32];
+            tmem_ld32(taddr + c * 32, x);
+            tmem_ld_wait();
+            const uint32_t dst = map_to_cta(slot_row, (uint32_t)(2 * owner) | rank) +
+                                 (uint32_t)((c / p.splits) * p.splits + split) * (HALF * 128u);
+#pragma unroll
+            for (int g = 0; g < 8; g++) st_cluster_v4(dst + (uint32_t)(g * HALF * 16), x[4 * g], x[4 * g + 1], x[4 * g + 2], x[4 * g + 3]);
+          }
+        }
+        __syncwarp();
+        cluster_sync_all();   // every slot has landed
+        if (!ok) break;
+      }
       if (ch0 < p.N) {
         uint32_t v[32];
-        if (part * 32 < p.np) tmem_ld32(taddr + part * 32, v);
+        // this warp's chunks: every PARTS-th one (SPLIT: of the pair's own)
+        const int c_first = SPLIT ? split + p.splits * part : part, c_step = SPLIT ? p.splits * PARTS : PARTS;
+        if (!SPLIT && c_first * 32 < p.np) tmem_ld32(taddr + c_first * 32, v);
 #pragma unroll 1
-        for (int c = part; c * 32 < p.np; c += PARTS) {
-          const int c_next = c + PARTS;
+        for (int c = c_first; c * 32 < p.np; c += c_step) {
+          const int c_next = c + c_step;
+          if constexpr (SPLIT) tmem_ld32(taddr + c * 32, v);
           // this lane's pixel of the chunk, worked out while the load is in flight
           const PixelRow px = pixel_row(p, (long long)tm * p.np + c * 32 + lane);
           tmem_ld_wait();
-          if constexpr (EPI != 0) {
-            if constexpr (EPI == 2) {
-              // accesses are 32 consecutive channels of one pixel; the 32 pixels' rows come from shared memory.  Integers
-              // become floats, and back, through the low mantissa bits of 1.5 * 2^23.
-              __syncwarp();
-              rows_s[32 + lane] = px.dense;
-              __syncwarp();
-              const int4* row4 = reinterpret_cast<const int4*>(rows_s) + 8;
-              constexpr float MAGIC = 12582912.0f;   // 1.5 * 2^23
-              if (ch < p.N && p.residual_in != nullptr) {
-                const int16_t* R = reinterpret_cast<const int16_t*>(p.residual_in) + ch;
-                auto add = [&](uint32_t& x, int r) {
-                  x = __float_as_uint(__uint_as_float(x) + (__int_as_float(0x4B400000 + r) - MAGIC));
-                };
+          if constexpr (SPLIT) {
+            for (int o = 0; o < p.splits; o++) {
+              if (o == split) continue;
+              const uint32_t src = slot_row + (uint32_t)((c / p.splits) * p.splits + o) * (HALF * 128u);
 #pragma unroll
-                for (int g = 0; g < 8; g++) {
-                  const int4 d = row4[g];
-                  add(v[4 * g], ld_row16(R, d.x, p.N));
-                  add(v[4 * g + 1], ld_row16(R, d.y, p.N));
-                  add(v[4 * g + 2], ld_row16(R, d.z, p.N));
-                  add(v[4 * g + 3], ld_row16(R, d.w, p.N));
-                }
-              }
-              if (ch < p.N && p.residual_out != nullptr) {
-                int16_t* R = reinterpret_cast<int16_t*>(p.residual_out) + ch;
-                auto sat = [](uint32_t x) {
-                  return __float_as_uint(fminf(fmaxf(__uint_as_float(x), -32768.0f), 32767.0f) + MAGIC);
-                };
-#pragma unroll
-                for (int g = 0; g < 8; g++) {
-                  const int4 d = row4[g];
-                  st_row16(R, d.x, p.N, sat(v[4 * g]));
-                  st_row16(R, d.y, p.N, sat(v[4 * g + 1]));
-                  st_row16(R, d.z, p.N, sat(v[4 * g + 2]));
-                  st_row16(R, d.w, p.N, sat(v[4 * g + 3]));
-                }
-              }
+              for (int g = 0; g < 8; g++) add_shared_v4(v + 4 * g, src + (uint32_t)(g * HALF * 16));
             }
-            const uint32_t b1 = below_bits(v, nt1), b2 = below_bits(v, nt2), b3 = below_bits(v, nt3);
-            if (c_next * 32 < p.np) tmem_ld32(taddr + c_next * 32, v);   // in flight during the rest of this chunk
-            // level = number of thresholds reached, as two bit words; then one word pair per pixel
-            const uint32_t p0 = __brev(transpose_bits(~(b1 ^ b2 ^ b3), lane));
-            const uint32_t p1 = __brev(transpose_bits(~((b1 & b2) | (b1 & b3) | (b2 & b3)), lane));
-            if (px.row >= 0) {
-              if (p.rows_out == 2) {
-                *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + (((long long)px.row * p.N + ch0) >> 1)) = nibbles_of(p0, p1);
-              } else if (p.rows_out == 1) {
-                uint32_t r[8];
-#pragma unroll
-                for (int q = 0; q < 8; q++) r[q] = ((p0 >> q) & 0x01010101u) | (((p1 >> q) & 0x01010101u) << 1);
-                store_32(reinterpret_cast<uint8_t*>(p.out) + (long long)px.row * p.N + ch0, r);
-              } else {
-                uint32_t* O = reinterpret_cast<uint32_t*>(p.out) + (long long)px.row * (p.N >> 5) + (ch0 >> 5);
-                O[0] = p0;
-                if (p.out_bits > 1) O[p.out_plane_words] = p1;
-              }
-            }
-            __syncwarp();
-          } else {
-            const bool ch_ok = ch < p.N;
-#pragma unroll
-            for (int j = 0; j < 32; j++) v[j] = (uint32_t)__float2int_rn(__uint_as_float(v[j]));
-            // every access below is 32 consecutive channels of one pixel; the 32 pixels' rows come from shared memory
-            __syncwarp();
-            rows_s[lane] = px.row;
-            rows_s[32 + lane] = px.dense;
-            __syncwarp();
-            const int4* row4 = reinterpret_cast<const int4*>(rows_s);
-            if (ch_ok && p.residual_in != nullptr) {
-              if (p.res16_in) {
-                const int16_t* R = reinterpret_cast<const int16_t*>(p.residual_in) + ch;
-#pragma unroll
-                for (int g = 0; g < 8; g++) {
-                  const int4 d = row4[8 + g];
-                  v[4 * g] += (uint32_t)ld_row16(R, d.x, p.N);
-                  v[4 * g + 1] += (uint32_t)ld_row16(R, d.y, p.N);
-                  v[4 * g + 2] += (uint32_t)ld_row16(R, d.z, p.N);
-                  v[4 * g + 3] += (uint32_t)ld_row16(R, d.w, p.N);
-                }
-              } else {
-                const int32_t* R = p.residual_in + ch;
-#pragma unroll
-                for (int g = 0; g < 8; g++) {
-                  const int4 d = row4[8 + g];
-                  v[4 * g] += (uint32_t)ld_row32(R, d.x, p.N);
-                  v[4 * g + 1] += (uint32_t)ld_row32(R, d.y, p.N);
-                  v[4 * g + 2] += (uint32_t)ld_row32(R, d.z, p.N);
-                  v[4 * g + 3] += (uint32_t)ld_row32(R, d.w, p.N);
-                }
-              }
-            }
-            if (ch_ok && p.residual_out != nullptr) {
-              if (p.res16_out) {
-                int16_t* R = reinterpret_cast<int16_t*>(p.residual_out) + ch;
-                auto sat = [](uint32_t x) { return (uint32_t)min(max((int)x, -32768), 32767); };
-#pragma unroll
-                for (int g = 0; g < 8; g++) {
-                  const int4 d = row4[8 + g];
-                  st_row16(R, d.x, p.N, sat(v[4 * g]));
-                  st_row16(R, d.y, p.N, sat(v[4 * g + 1]));
-                  st_row16(R, d.z, p.N, sat(v[4 * g + 2]));
-                  st_row16(R, d.w, p.N, sat(v[4 * g + 3]));
-                }
-              } else {
-                int32_t* R = p.residual_out + ch;
-#pragma unroll
-                for (int g = 0; g < 8; g++) {
-                  const int4 d = row4[8 + g];
-                  st_row32(R, d.x, p.N, v[4 * g]);
-                  st_row32(R, d.y, p.N, v[4 * g + 1]);
-                  st_row32(R, d.z, p.N, v[4 * g + 2]);
-                  st_row32(R, d.w, p.N, v[4 * g + 3]);
-                }
-              }
-            }
-            if (p.out_mode == OUT_INT32) {
-              int32_t* D = reinterpret_cast<int32_t*>(p.out) + ch;
-              if (ch_ok) {
-#pragma unroll
-                for (int g = 0; g < 8; g++) {
-                  const int4 d = row4[g];
-                  st_row32(D, d.x, p.N, v[4 * g]);
-                  st_row32(D, d.y, p.N, v[4 * g + 1]);
-                  st_row32(D, d.z, p.N, v[4 * g + 2]);
-                  st_row32(D, d.w, p.N, v[4 * g + 3]);
-                }
-              }
-            } else {
-              // packed modes need N % 32 == 0: all 32 channels of the warp exist
-              if (p.out_mode == OUT_THRESHOLDS) {
-                uint32_t lv[32];
-#pragma unroll
-                for (int j = 0; j < 32; j++) lv[j] = 0u;
-                const int32_t* T = p.thresholds + (long long)ch * nl;
-#pragma unroll 1
-                for (int t = 0; t < nl; t++) {
-                  const int thr = __ldg(T + t);
-#pragma unroll
-                  for (int j = 0; j < 32; j++) lv[j] += ((int)v[j] >= thr) ? 1u : 0u;
-                }
-#pragma unroll
-                for (int j = 0; j < 32; j++) v[j] = lv[j];
-              }
-              uint32_t r[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-              uint32_t first = 0u, second = 0u;
-#pragma unroll 1
-              for (int b = 0; b < p.out_bits; b++) {
-                uint32_t w = 0u;
-#pragma unroll
-                for (int j = 0; j < 32; j++) w |= ((v[j] >> b) & 1u) << j;
-                const uint32_t plane = __brev(transpose_bits(w, lane));
-                if (p.rows_out == 1) {
-#pragma unroll
-                  for (int q = 0; q < 8; q++) r[q] |= ((plane >> q) & 0x01010101u) << b;
-                } else if (p.rows_out == 2) {
-                  if (b == 0) first = plane;
-                  else second = plane;
-                } else if (px.row >= 0) {
-                  reinterpret_cast<uint32_t*>(p.out)[b * p.out_plane_words + (long long)px.row * (p.N >> 5) + (ch0 >> 5)] = plane;
-                }
-              }
-              if (px.row >= 0) {
-                if (p.rows_out == 1) store_32(reinterpret_cast<uint8_t*>(p.out) + (long long)px.row * p.N + ch0, r);
-                else if (p.rows_out == 2)
-                  *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + (((long long)px.row * p.N + ch0) >> 1)) =
-                      nibbles_of(first, second);
-              }
-            }
-            __syncwarp();   // lanes that skipped a store rejoin before the warp-wide TMEM load
-            if (c_next * 32 < p.np) tmem_ld32(taddr + c_next * 32, v);
           }
+          finish_chunk<EPI>(p, v, px, lane, ch0, thr, nl, rows_s, [&] {
+            if (!SPLIT && c_next * 32 < p.np) tmem_ld32(taddr + c_next * 32, v);
+          });
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), 0));   // the leader's barrier
+      if (lane == 0) mbar_arrive_cluster(map_to_cta(tempty_bar(acc), leader));   // the leader's barrier
     }
     if (!ok && lane == 0) atomicExch(p.error_flag, 3);
   }
@@ -600,7 +348,7 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   tc_fence_before();
   __syncthreads();
   grid_launch_dependents();   // the next kernel of the stream may start its prologue
-  cluster_sync_all();         // the peer may not leave while the leader's MMAs or arrivals can still reach it
+  cluster_sync_all();         // the peer (SPLIT: the cluster) may not leave while the leader's MMAs or arrivals can still reach it
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512));
@@ -624,44 +372,50 @@ bool make_rows_map(CUtensorMap* map, const void* base, long long rows, long long
             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// floor(n / d) == (n * magic) >> shift for every 0 <= n < 2^31 (d >= 1): with L = ceil(log2 d),
-// magic = floor(2^(31+L) / d) + 1 and shift = 31 + L; magic <= 2^32, the product stays below 2^63.
-void division_magic(int d, unsigned long long* magic, int* shift) {
-  int L = 0;
-  while ((1ll << L) < d) L++;
-  *shift = 31 + L;
-  *magic = ((1ull << (31 + L)) / (unsigned long long)d) + 1ull;
-}
-
 int box_rows_of(int R, int Wp, int np) { return (np / 2 + (R - 1) * (Wp + 1) + 7) / 8 * 8; }
 
 struct Fp4Plan {
   int np;          // 0: not applicable
+  int splits;      // pairs of a cluster that share a tile's K
   long long clk;   // estimated SM clocks
 };
-// Tile width: waves x (MMAs of a tile, or the filter bytes they need at the rate L2 delivers, whichever is longer) plus
-// the set-up and the last tile's epilogue.  Widths are multiples of 32 (whole epilogue chunks), the pixel box at most 256 rows.
+int fp4_cluster_capacity(int splits, int span);
+
+// Tile width and K split: waves x (MMAs of a tile, or its operand bytes at the rate L2 delivers, whichever is longer; or
+// its epilogue) plus the set-up, the last tile's epilogue and the exchange of a split.  Widths are multiples of 32 (whole
+// epilogue chunks), the pixel box at most 256 rows; a split problem is one wave of resident clusters, and is taken when it
+// saves a tenth.
 Fp4Plan plan_np(long long flat_rows, int COUT, int R, int Wp, int kbytes_per_tap, int span, int sms) {
-  Fp4Plan best = {0, 0};
-  const long long taps = (long long)R * R * (kbytes_per_tap / span);   // filter tiles of `span` bytes
+  Fp4Plan best = {0, 1, 0};
+  const long long cblocks = kbytes_per_tap / span;
   const long long tiles_n = (COUT + TILE_CH - 1) / TILE_CH;
   const int pairs = sms / 2;
-  for (int np = MAX_NP; np >= 32; np -= 32) {
-    const int rows = box_rows_of(R, Wp, np);
-    if (rows > 256) continue;
-    const long long tiles = ((flat_rows + np - 1) / np) * tiles_n;
-    const long long waves = (tiles + pairs - 1) / pairs;
-    const long long mma = taps * np * 2 * span / 128;
-    const long long feed = (taps * HALF * span + (long long)(kbytes_per_tap / span) * rows * span) / 54;
-    const long long epi = 9LL * np;   // measured: about 2000 clk for 224 pixels
-    const long long per = mma > feed ? mma : feed;
-    const long long clk = waves * (per > epi ? per : epi) + epi + 6000;
-    if (best.np == 0 || clk < best.clk) best = {np, clk};
+  for (int splits = 1; splits <= 4 && splits * 2 <= cblocks + (splits == 1 ? 1 : 0); splits *= 2) {
+    Fp4Plan here = {0, splits, 0};
+    for (int np = MAX_NP; np >= 32; np -= 32) {
+      const int rows = box_rows_of(R, Wp, np);
+      if (rows > 256) continue;
+      const long long tiles = ((flat_rows + np - 1) / np) * tiles_n;
+      if (splits > 1 && (tiles * splits > pairs || tiles > fp4_cluster_capacity(splits, span))) continue;
+      const long long waves = (tiles + pairs - 1) / pairs;
+      const long long kb = (cblocks + splits - 1) / splits;   // K blocks of one pair
+      const long long mma = kb * R * R * np * 2 * span / 128;
+      const long long feed = kb * span * ((long long)R * R * HALF + rows) / 54;
+      const long long epi = 9LL * np;   // measured: about 2000 clk for 224 pixels
+      long long per = mma > feed ? mma : feed;
+      if (splits > 1) {   // one wave that streams the filter: about 3900 B/clk over the chip (7.3 TB/s, little L2 reuse)
+        const long long stream = ((flat_rows + np - 1) / np) * COUT * R * R * kbytes_per_tap / 3900;
+        if (per < stream) per = stream;
+      }
+      const long long clk = waves * (per > epi ? per : epi) + epi / splits + 6000 + (splits > 1 ? 2000 : 0);
+      if (here.np == 0 || clk < here.clk) here = {np, splits, clk};
+    }
+    if (here.np && (best.np == 0 || here.clk * 10 <= best.clk * 9)) best = here;
   }
   return best;
 }
 
-template <int RR, int BKB, int EPI>
+template <int RR, int BKB, int EPI, bool SPLIT>
 cudaError_t launch_fp4(cudaStream_t s, const CUtensorMap& map_x, const CUtensorMap& map_w, Fp4Params& p, int pairs) {
   constexpr int stage = RR * HALF * BKB;
   // ring depths: filter stages take what two pixel boxes leave (one tap: as many boxes as filter tiles)
@@ -679,7 +433,7 @@ cudaError_t launch_fp4(cudaStream_t s, const CUtensorMap& map_x, const CUtensorM
     if (na > 4) na = 4;
   }
   if (na < 1 || nb < 2) return cudaErrorInvalidConfiguration;
-  p.w_resident = p.tiles_n == 1 && p.cblocks == 1 && nb >= RR;
+  p.w_resident = !SPLIT && p.tiles_n == 1 && p.cblocks == 1 && nb >= RR;
   if (p.w_resident) {   // stage ti of every tile is slot ti; the boxes get the rest
     nb = RR;
     na = (room - nb * stage) / (int)p.a_buf;
@@ -687,23 +441,73 @@ cudaError_t launch_fp4(cudaStream_t s, const CUtensorMap& map_x, const CUtensorM
   }
   p.na = na;
   p.nb = nb;
-  const int smem = 1024 + BAR_BYTES + ROWS_BYTES + na * (int)p.a_buf + nb * stage;
-  cudaError_t e = ensure_max_smem(reinterpret_cast<const void*>(tc5_conv_fp4_kernel<RR, BKB, EPI>), SMEM_LIMIT);
+  int ring = na * (int)p.a_buf + nb * stage;
+  const int exchange = SPLIT ? (p.np / 32 + p.splits - 1) / p.splits * p.splits * HALF * 128 : 0;
+  if (ring < exchange) ring = exchange;
+  if (ring > room) return cudaErrorInvalidConfiguration;
+  p.ring_bytes = (uint32_t)ring;
+  const int smem = 1024 + BAR_BYTES + ROWS_BYTES + (int)p.ring_bytes;
+  cudaError_t e = ensure_max_smem(reinterpret_cast<const void*>(tc5_conv_fp4_kernel<RR, BKB, EPI, SPLIT>), SMEM_LIMIT);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(2 * pairs, 1, 1);
+  cfg.gridDim = dim3(2 * pairs * (SPLIT ? p.splits : 1), 1, 1);
   cfg.blockDim = dim3(threads_of(EPI, BKB), 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = SPLIT ? 2 * p.splits : 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1 + (unsigned)pdl_attribute(attr + 1);
-  return cudaLaunchKernelEx(&cfg, tc5_conv_fp4_kernel<RR, BKB, EPI>, map_x, map_w, p);
+  return cudaLaunchKernelEx(&cfg, tc5_conv_fp4_kernel<RR, BKB, EPI, SPLIT>, map_x, map_w, p);
+}
+
+// How many clusters of `splits` pairs the device holds at once (0 on error); cached per device.
+int fp4_cluster_capacity(int splits, int span) {
+  static std::mutex mu;
+  static int cache[16][2][2] = {};   // value + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 16 || (splits != 2 && splits != 4)) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  int& slot = cache[dev][splits == 4][span == 64];
+  if (slot) return slot - 1;
+  const void* kernel = span == 128 ? reinterpret_cast<const void*>(tc5_conv_fp4_kernel<1, 128, 1, true>)
+                                   : reinterpret_cast<const void*>(tc5_conv_fp4_kernel<1, 64, 1, true>);
+  int n = 0;
+  if (ensure_max_smem(kernel, SMEM_LIMIT) == cudaSuccess) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(2 * splits * device_sm_count()), 1, 1);
+    cfg.blockDim = dim3(threads_of(1, span), 1, 1);
+    cfg.dynamicSmemBytes = SMEM_LIMIT;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)(2 * splits);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+  }
+  slot = n + 1;
+  return n;
+}
+
+template <int RR, int SPAN>
+cudaError_t launch_kind(cudaStream_t s, const CUtensorMap& map_x, const CUtensorMap& map_w, Fp4Params& p, int pairs, int kind) {
+  if (p.splits > 1) {   // residuals of a split problem take the general epilogue
+    if (kind == 1) return launch_fp4<RR, SPAN, 1, true>(s, map_x, map_w, p, pairs);
+    return launch_fp4<RR, SPAN, 0, true>(s, map_x, map_w, p, pairs);
+  }
+  if (kind == 1) return launch_fp4<RR, SPAN, 1, false>(s, map_x, map_w, p, pairs);
+  if (kind == 2) return launch_fp4<RR, SPAN, 2, false>(s, map_x, map_w, p, pairs);
+  return launch_fp4<RR, SPAN, 0, false>(s, map_x, map_w, p, pairs);
 }
 
 }  // namespace
@@ -752,17 +556,13 @@ apnn_status tc5_conv_fp4(cudaStream_t s, const uint8_t* X4, const uint8_t* W4, v
     p.residual_out = epi->residual_out;
     p.out_bits = epi->out_bits;
     p.rows_out = epi->out_i8;
+    p.affine_scale = epi->affine_scale;
+    p.affine_bias = epi->affine_bias;
     p.res16_in = epi->residual_i16 & 1;
     p.res16_out = (epi->residual_i16 >> 1) & 1;
   }
-  p.wp = Wp;
-  p.hpwp = Hp * Wp;
-  division_magic(p.hpwp, &p.magic_hpwp, &p.shift_hpwp);
-  division_magic(p.wp, &p.magic_wp, &p.shift_wp);
+  set_image(p, B, Hin, Win, Hp, Wp);
   p.in_off = in_halo - pad;
-  p.Bn = B;
-  p.Ho = Hin;
-  p.Wo = Win;
   p.a_bytes = (uint32_t)(box_rows * span);
   p.a_buf = (p.a_bytes + 1023u) & ~1023u;
   p.error_flag = status_flag;
@@ -777,15 +577,18 @@ apnn_status tc5_conv_fp4(cudaStream_t s, const uint8_t* X4, const uint8_t* W4, v
   const bool all16 = (!p.residual_in || p.res16_in) && (!p.residual_out || p.res16_out);
   const int kind = thr2 && !residuals ? 1 : thr2 && all16 && 9LL * R * R * CIN + 32768 < (1ll << 24) ? 2 : 0;
   cudaError_t e;
-#define APNN_FP4_CASE(RR, SPAN) \
-  (kind == 1   ? launch_fp4<RR, SPAN, 1>(s, map_x, map_w, p, pairs) \
-   : kind == 2 ? launch_fp4<RR, SPAN, 2>(s, map_x, map_w, p, pairs) \
-               : launch_fp4<RR, SPAN, 0>(s, map_x, map_w, p, pairs))
-  if (R == 3) e = span == 128 ? APNN_FP4_CASE(3, 128) : APNN_FP4_CASE(3, 64);
-  else e = span == 128 ? APNN_FP4_CASE(1, 128) : APNN_FP4_CASE(1, 64);
-#undef APNN_FP4_CASE
+  p.splits = pl.splits;
+  if (R == 3) e = span == 128 ? launch_kind<3, 128>(s, map_x, map_w, p, pairs, kind) : launch_kind<3, 64>(s, map_x, map_w, p, pairs, kind);
+  else e = span == 128 ? launch_kind<1, 128>(s, map_x, map_w, p, pairs, kind) : launch_kind<1, 64>(s, map_x, map_w, p, pairs, kind);
   if (e != cudaSuccess) return cuda_fail(e, "tc5_conv_fp4 launch");
   return APNN_OK;
+}
+
+// D[m][n] over nibble rows A4 [M][K/2], B4 [N][K/2]: one tap, the rows of A as pixels and the rows of B as channels.
+long long tc5_gemm_fp4_flat_clocks(int M, int N, int K) { return tc5_conv_fp4_clocks(1, 1, M, K, N, 1, 0, 0); }
+apnn_status tc5_gemm_fp4_flat(cudaStream_t s, const uint8_t* A4, const uint8_t* B4, void* D, int M, int N, int K,
+                              const apnn_epilogue* epi, int* status_flag) {
+  return tc5_conv_fp4(s, A4, B4, D, 1, 1, M, K, N, 1, epi, status_flag);
 }
 
 }  // namespace apnn

@@ -1633,6 +1633,18 @@ apnn_status tc5_gemm(cudaStream_t s, int wbits, int xbits, const uint32_t* W, co
     if (s4 != APNN_OK) return s4;
     return tc5_gemm_fp4_pair(s, wa, xb4, D, M, N, K, epi, err);
   }
+  // problems with fewer tiles than that: the flat 4-bit kernel, whose tile width and K split follow the shape, for the
+  // two-bit thresholds it packs cheaply (128 x 4096 x 9216: 18.3 us against 22.1 on int8; 2048^3 16.3 / 15.1, 1024 x 1024 x
+  // 2048 11.2 / 12.9; int32 rows 2048^3 17.9 / 13.6)
+  const bool thr2 = epi && epi->out_mode == APNN_OUT_THRESHOLDS && epi->out_bits <= 2 && !epi->residual_in && !epi->residual_out &&
+                    epi->n_peer_out == 0;
+  if (fp4_on && wbits <= 2 && xbits <= 2 && !pair && thr2 && !takes_pair_kernel(M, N, K, epi) &&
+      tc5_gemm_fp4_flat_clocks(M, N, K) != 0) {
+    uint8_t* xb4 = wa + align_up((size_t)M * (K / 2), 256);
+    apnn_status s4 = tc5_expand2_fp4(s, W, wa, M, wbits, sign == APNN_SIGN_W, X, xb4, N, xbits, sign == APNN_SIGN_X, K);
+    if (s4 != APNN_OK) return s4;
+    return tc5_gemm_fp4_flat(s, wa, xb4, D, M, N, K, epi, err);
+  }
   // APNN_XPLANES=1: the CTA-pair kernel spreads the activation planes itself, so only W goes through the expand
   // pass and the activation part of the workspace stays untouched.  Off by default: at 8192^3 that kernel takes
   // 0.45 ms against 0.017 + 0.288 ms for the expand pass and the GEMM over int8 rows.

@@ -41,11 +41,15 @@ apnn_status tc5_expand_fp4(cudaStream_t s, const uint32_t* planes, uint8_t* out,
                            bool is_signed);
 apnn_status tc5_expand2_fp4(cudaStream_t s, const uint32_t* pa, uint8_t* oa, long long rows_a, int bits_a, bool signed_a,
                             const uint32_t* pb, uint8_t* ob, long long rows_b, int bits_b, bool signed_b, int K);
-// Stride-1 convolution over e2m1 nibble rows (tc5_fp4.cu): R in {1, 3}, CIN % 128 == 0, no pooling, any output mode but
-// float; epi->out_i8 = 2 writes nibble rows.  The estimate is in SM clocks, 0 for shapes it does not take.
+// Stride-1 convolution over e2m1 nibble rows (tc5_fp4.cu): R in {1, 3}, CIN % 128 == 0, no pooling, any output mode;
+// epi->out_i8 = 2 writes nibble rows.  The estimate is in SM clocks, 0 for shapes it does not take.
 long long tc5_conv_fp4_clocks(int B, int H, int W, int CIN, int COUT, int R, int in_halo, int out_halo);
 apnn_status tc5_conv_fp4(cudaStream_t s, const uint8_t* X4, const uint8_t* W4, void* Out, int B, int H, int W, int CIN,
                          int COUT, int R, const apnn_epilogue* epi, int* status_flag);
+// The GEMM on the same kernel (any M and N, K % 128 == 0): narrow tiles and split K for problems of few tiles.
+long long tc5_gemm_fp4_flat_clocks(int M, int N, int K);
+apnn_status tc5_gemm_fp4_flat(cudaStream_t s, const uint8_t* A4, const uint8_t* B4, void* D, int M, int N, int K,
+                              const apnn_epilogue* epi, int* status_flag);
 apnn_status tc5_gemm_fp4_pair(cudaStream_t s, const uint8_t* A4, const uint8_t* B4, void* D, int M, int N, int K,
                               const apnn_epilogue* epi, int* status_flag);
 // The flat convolution on CTA pairs (256 positions x 256 channels per pair): stride 1, no pooling,

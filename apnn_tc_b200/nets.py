@@ -497,9 +497,12 @@ class Network:
         with residuals stay on int8, whose epilogue fetches them ahead (1024 x 14x14, 256 channels: 115 us against 123)."""
         if ls.residual_from or ls.save_residual:
             return False
-        if ls.kind != "conv" or not self.i8_out.get(self.src_of[ls.name], False) or ls.stride != 1 or ls.R not in (1, 3):
-            return False
         sh = self.params[ls.name].shape
+        if ls.kind != "conv":      # fully connected: half the weight bytes to stream, whatever the shape
+            return (self.i8_out.get(self.src_of[ls.name], False) and self.spec.a_bit <= 2 and self.spec.w_bit == 1
+                    and 9 * sh["K"] < 2 ** 24)
+        if not self.i8_out.get(self.src_of[ls.name], False) or ls.stride != 1 or ls.R not in (1, 3):
+            return False
         ring = self.halo[self.src_of[ls.name]]
         return (self.spec.a_bit <= 2 and self.spec.w_bit == 1 and sh["cinp"] % 128 == 0 and sh["coutp"] >= 256
                 and 9 * ls.R * ls.R * sh["cinp"] < 2 ** 24 and (ls.R == 1 or sh["W"] + 2 * ring <= 100)
@@ -515,7 +518,9 @@ class Network:
             return
         users = {ls.name: [c for c in self.spec.layers if self.src_of[c.name] == ls.name] for ls in self.spec.layers}
         for ls in self.spec.layers:
-            if ls.kind == "conv" and self.i8_out.get(ls.name, False) and all(self._fp4_candidate(u) for u in users[ls.name]):
+            # (a fully connected layer writes nibbles when it runs on them itself)
+            if (self.i8_out.get(ls.name, False) and (ls.kind == "conv" or self.fp4.get(ls.name, False))
+                    and all(self._fp4_candidate(u) for u in users[ls.name])):
                 self.fp4_out[ls.name] = True
                 for u in users[ls.name]:
                     wp = self.w_planes[u.name]
@@ -637,6 +642,10 @@ class Network:
         epi = self._epilogue(ls, False)
         out = self.out[ls.name]
         s = _stream_ptr()
+        if self.fp4.get(ls.name, False):
+            _cabi.check(self.L.apnn_linear_fp4(s, X.data_ptr(), self.w4[ls.name].data_ptr(), out.data_ptr(), B, N, K,
+                                               ctypes.byref(epi), self.flag.data_ptr()), "apnn_linear_fp4 " + ls.name)
+            return 1
         if self.tc5_ok[ls.name]:
             n, x8 = 1, X
             if not self.i8_out.get(self.src_of[ls.name], False):

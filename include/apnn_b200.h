@@ -271,6 +271,10 @@ apnn_status apnn_conv2d_i8(void *stream, const void *W8, const void *X8, void *O
 apnn_status apnn_conv2d_fp4(void *stream, const void *W4, const void *X4, void *Out, int B, int H, int W,
                             int CIN, int COUT, int R, const apnn_epilogue *epi, int *status_flag);
 
+/* The fully connected layer on the same kernel: Out[m][n] over nibble rows X4[M][K/2] (activations) and W4[N][K/2]
+ * (weights), K % 128 == 0, 9*K < 2^24; every output mode (APNN_OUT_FLOAT and row forms as above included). */
+apnn_status apnn_linear_fp4(void *stream, const void *X4, const void *W4, void *Out, int M, int N, int K,
+                            const apnn_epilogue *epi, int *status_flag);
 /* apnn_conv2d_i8 (int8 operands) whose quantised output leaves as e2m1 nibble rows: epi->out_i8 = APNN_ROWS_FP4. */
 apnn_status apnn_conv2d_i8_to_fp4(void *stream, const void *W8, const void *X8, void *Out, int B, int H, int W,
                                   int CIN, int COUT, int R, int stride, int w_signed,

@@ -171,3 +171,52 @@ def test_int8_layer_writes_nibble_rows(cuda_device, CIN, COUT, R, stride, mode, 
     want = np.full(out.shape, 0xEE, dtype=np.uint8)
     want[:, halo:-halo, halo:-halo] = spread_nibbles(lv)
     assert np.array_equal(out.cpu().numpy(), want) and int(flag.item()) == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 32, 128), (128, 4096, 2304), (64, 512, 9216), (200, 96, 1280), (33, 1000, 4096), (8, 512, 25088),
+                                   (2300, 352, 640)])
+@pytest.mark.parametrize("sign", ["none", "w", "x"])
+def test_gemm_on_narrow_tiles_and_split_k(cuda_device, M, N, K, sign):
+    """apnn_linear_fp4 (split K, ragged edges, every output form) and apmm on tcgen05 below the CTA-pair kernel's size."""
+    import apnn_tc_b200 as ap
+    from apnn_tc_b200 import _cabi
+    from apnn_tc_b200.ops import _stream_ptr
+    rng = np.random.default_rng(M + N + K)
+    wb, xb = (1, 2) if sign == "w" else (2, 1) if sign == "x" else (2, 2)
+    W, _ = oracle.value_planes(rng, M, K, wb)
+    X, _ = oracle.value_planes(rng, N, K, xb)
+    v = oracle.gemm_popc(W, X, threads=8)
+    if sign == "w":
+        v = oracle.signed_correct(v, oracle.row_sums(X), 1)
+    elif sign == "x":
+        v = oracle.signed_correct(v, oracle.row_sums(W), 0)
+    ws = torch.empty(ap.gemm_workspace_bytes(M, N, K), dtype=torch.uint8, device="cuda")
+    epi = ap.make_epilogue("int32", signed=sign)
+    assert np.array_equal(to_host(ap.apmm(to_dev(W), to_dev(X), epilogue=epi, algo="tcgen05", workspace=ws), np.int32), v)
+    ap.gemm_check(ws, M, N, K)
+    T = np.sort(rng.integers(int(v.min()) - 1, int(v.max()) + 2, size=(N, 3)), axis=1).astype(np.int32)
+    x4, w4 = expand(W, sign == "w"), expand(X, sign == "x")
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def linear(out, e):
+        _cabi.check(_cabi.lib().apnn_linear_fp4(_stream_ptr(), x4.data_ptr(), w4.data_ptr(), out.data_ptr(), M, N, K,
+                                                ctypes.byref(e), flag.data_ptr()), "apnn_linear_fp4")
+        assert int(flag.item()) == 0
+        return out
+    got = linear(torch.zeros((M, N), dtype=torch.int32, device="cuda"), ap.make_epilogue("int32"))
+    assert np.array_equal(to_host(got, np.int32), v)
+    sc, bi = rng.uniform(0.5, 1.5, N).astype(np.float32), rng.uniform(-1, 1, N).astype(np.float32)
+    e = ap.make_epilogue("float", affine_scale=torch.from_numpy(sc).cuda(), affine_bias=torch.from_numpy(bi).cuda())
+    got = linear(torch.zeros((M, N), dtype=torch.float32, device="cuda"), e).cpu().numpy()
+    assert np.array_equal(got, oracle.affine_f32(v, sc, bi))
+    if N % 32:
+        return
+    for mode, bits in (("thresholds", 2), ("lowbits", 2), ("lowbits", 5)):
+        epi = ap.make_epilogue(mode, bits, signed=sign, thresholds=to_dev(T))
+        want = oracle.requant_pack(v, bits, 2 if mode == "thresholds" else 1, T)
+        assert np.array_equal(to_host(ap.apmm(to_dev(W), to_dev(X), epilogue=epi, algo="tcgen05", workspace=ws)), want)
+    lv = oracle.levels(v, 2, 2, T)
+    for form in (1, 2):
+        out = linear(torch.zeros((M, N // form), dtype=torch.uint8, device="cuda"),
+                     ap.make_epilogue("thresholds", 2, thresholds=to_dev(T), out_i8=form)).cpu().numpy()
+        assert np.array_equal(out, spread_bytes(lv) if form == 1 else spread_nibbles(lv))
