@@ -26,7 +26,7 @@ EXPORTS = (
     "apnn_gemm_workspace_bytes", "apnn_gemm_check", "apnn_expand_planes", "apnn_expand_planes_pair", "apnn_gemm_i8", "apnn_gemm_w8", "apnn_expand_planes_fp4", "apnn_gemm_fp4", "apnn_gemm_static_scratch", "apnn_conv2d", "apnn_conv2d_ex",
     "apnn_conv2d_workspace_bytes", "apnn_conv2d_check", "apnn_conv2d_i8", "apnn_bit_compress", "apnn_quantize_pack", "apnn_quantize_im2col", "apnn_create",
     "apnn_destroy", "apnn_gemm_host", "apnn_conv2d_host", "apnn_probe_peak", "apnn_quantize_im2col_i8", "apnn_quantize_window_rows_i8", "apnn_quantize_blocks_i8", "apnn_maxpool2x2_i8", "apnn_requantize_i32",
-    "apnn_conv2d_fp4", "apnn_linear_fp4", "apnn_conv2d_i8_to_fp4", "apnn_maxpool2x2_rows",
+    "apnn_conv2d_fp4", "apnn_linear_fp4", "apnn_gemm_planes", "apnn_conv2d_i8_to_fp4", "apnn_maxpool2x2_rows",
 )
 
 
@@ -106,6 +106,7 @@ def lib() -> ctypes.CDLL:
     L.apnn_quantize_blocks_i8.argtypes = [vp, vp, vp, i, i, i, i, i, i, i, i]
     L.apnn_maxpool2x2_i8.argtypes = [vp, vp, vp, i, i, i, i, i, i]
     L.apnn_conv2d_i8_to_fp4.argtypes = L.apnn_conv2d_i8.argtypes
+    L.apnn_gemm_planes.argtypes = [vp, i, i, vp, vp, vp, i, i, i, ep, vp]
     L.apnn_linear_fp4.argtypes = [vp, vp, vp, vp, i, i, i, ep, vp]
     L.apnn_conv2d_fp4.argtypes = [vp, vp, vp, vp, i, i, i, i, i, i, ep, vp]
     L.apnn_maxpool2x2_rows.argtypes = [vp, vp, vp, i, i, i, i, i, i, i, i]

@@ -239,8 +239,17 @@ apnn_status apnn_gemm_ex(void* stream, int algo, int wbits, int xbits, const voi
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 
   if (algo == APNN_ALGO_AUTO) {
-    bool ws_ok = workspace && workspace_bytes >= tc5_workspace_bytes(M, N, K);
-    algo = (ws_ok && (tc5_worthwhile(M, N, K) || !warp_ok)) ? APNN_ALGO_TCGEN05 : APNN_ALGO_IMMA;
+    const bool ws_ok = workspace && workspace_bytes >= tc5_workspace_bytes(M, N, K);
+    // operands of at most two bits, one wave of tiles: straight from the planes in one launch
+    if (ws_ok && !(epi && epi->n_peer_out != 0) &&
+        tc5_gemm_planes_preferred(wbits, xbits, M, N, K, epi && epi->out_mode != APNN_OUT_INT32))
+      return tc5_gemm_planes(s, wbits, xbits, (const uint32_t*)W, (const uint32_t*)X, D, M, N, K, epi,
+                             tc5_flag_slot(workspace, M, N, K));
+    // the expand pass and the tcgen05 kernels: many tiles, or two gigaoperations that are not a skinny problem, whose wide
+    // operand the expand pass would write and read for few uses (int32, us: 2048 x 2048 x 256 8.3 against 12.2 on the
+    // warp-level kernel, packed output 11.5 / 27.2; 8192 x 512 x 512 9.3 / 12.1; but 64 x 4096 x 4096 14.3 / 9.5)
+    const bool big = tc5_worthwhile(M, N, K) || (M >= 512 && N >= 512 && 2.0 * M * N * K >= 2e9);
+    algo = (ws_ok && (big || !warp_ok)) ? APNN_ALGO_TCGEN05 : APNN_ALGO_IMMA;
   }
   if (!warp_ok && algo != APNN_ALGO_TCGEN05 && algo != APNN_ALGO_TCGEN05_PAIR)
     return workspace ? APNN_ERR_UNSUPPORTED : APNN_ERR_WORKSPACE;
@@ -355,6 +364,17 @@ apnn_status apnn_conv2d_fp4(void* stream, const void* W4, const void* X4, void* 
   if (tc5_conv_fp4_clocks(B, H, W, CIN, COUT, R, in_halo, out_halo) == 0) return APNN_ERR_UNSUPPORTED;
   return tc5_conv_fp4(reinterpret_cast<cudaStream_t>(stream), (const uint8_t*)X4, (const uint8_t*)W4, Out, B, H, W, CIN, COUT,
                       R, epi, status_flag);
+}
+
+apnn_status apnn_gemm_planes(void* stream, int wbits, int xbits, const void* W, const void* X, void* D, int M, int N, int K,
+                             const apnn_epilogue* epi, int* status_flag) {
+  if (!W || !X || !D || !status_flag || M <= 0 || N <= 0 || K <= 0) return APNN_ERR_INVALID_ARG;
+  if (K % 128 != 0 || !aligned16(W) || !aligned16(X) || !aligned16(D)) return APNN_ERR_ALIGNMENT;
+  apnn_status st = check_epilogue(epi, N, false, wbits, xbits);
+  if (st != APNN_OK) return st;
+  if ((epi && epi->n_peer_out != 0) || tc5_gemm_planes_clocks(wbits, xbits, M, N, K) == 0) return APNN_ERR_UNSUPPORTED;
+  return tc5_gemm_planes(reinterpret_cast<cudaStream_t>(stream), wbits, xbits, (const uint32_t*)W, (const uint32_t*)X, D, M, N,
+                         K, epi, status_flag);
 }
 
 apnn_status apnn_linear_fp4(void* stream, const void* X4, const void* W4, void* Out, int M, int N, int K,

@@ -121,13 +121,12 @@ __device__ __forceinline__ unsigned long long negated2(float t) {
 // Level words of one pixel (bit 31 - c = channel c of the 32-channel group, one word per bit) -> the pixel's 16 bytes of
 // e2m1 nibbles, in expand_nibbles_kernel's order: nibble i of word q holds the element at bit 4i + q.
 __device__ __forceinline__ uint4 nibbles_of(uint32_t p0, uint32_t p1) {
-  uint32_t o[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const uint32_t t0 = (p0 >> q) & 0x11111111u, t1 = (p1 >> q) & 0x11111111u;
-    o[q] = (t1 << 2) | ((t0 & ~t1) << 1) | (t0 & t1);
-  }
-  return make_uint4(o[0], o[1], o[2], o[3]);
+  // code bits: 0 = both, 1 = the low bit alone, 2 = the high bit; each plane is shifted once per word and masked in place
+  constexpr uint32_t M = 0x11111111u;
+  const uint32_t a = p0 & p1, c = p0 & ~p1;
+  return make_uint4((a & M) | ((c << 1) & (M << 1)) | ((p1 << 2) & (M << 2)), ((a >> 1) & M) | (c & (M << 1)) | ((p1 << 1) & (M << 2)),
+                    ((a >> 2) & M) | ((c >> 1) & (M << 1)) | (p1 & (M << 2)),
+                    ((a >> 3) & M) | ((c >> 2) & (M << 1)) | ((p1 >> 1) & (M << 2)));
 }
 __device__ __forceinline__ void store_32(uint8_t* dst, const uint32_t (&r)[8]) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]),

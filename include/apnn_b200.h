@@ -204,6 +204,12 @@ apnn_status apnn_expand_planes_fp4(void *stream, const void *planes, void *out_f
 apnn_status apnn_gemm_fp4(void *stream, const void *W4, const void *X4, void *D, int M, int N, int K,
                           const apnn_epilogue *epi, int *status_flag);
 
+/* apnn_gemm_ex on the same tensor path in ONE launch, straight from the packed planes (wbits, xbits <= 2, K % 128 == 0,
+ * 9*K < 2^24; any M and N; no peer_out): the kernel spreads the bits into its operand stages itself.  For small and medium
+ * problems, which apnn_gemm_ex sends here by itself when it is given a workspace. */
+apnn_status apnn_gemm_planes(void *stream, int wbits, int xbits, const void *W, const void *X, void *D, int M, int N,
+                             int K, const apnn_epilogue *epi, int *status_flag);
+
 /* A tcgen05 GEMM that allocates nothing and needs no workspace argument.  No counterpart
  * in the reference.  It exists for callers that cannot cudaMalloc a workspace: code running
  * inside a host application whose own memory pool already owns the device's memory, or a
