@@ -442,7 +442,8 @@ long long tc5_gemm_planes_clocks(int wbits, int xbits, int M, int N, int K) {
 // For int32 the warp-level kernel, about 3.2 us + 1.5 us per 1024 k and wave of its 64 x 32 tiles, keeps the smallest
 // (64 x 1024 x 1024: 5.2 / 4.5; 1024 x 1024 x 512: 4.9 / 5.6).
 bool tc5_gemm_planes_preferred(int wbits, int xbits, int M, int N, int K, bool packed_out) {
-  if (tc5_gemm_planes_clocks(wbits, xbits, M, N, K) == 0) return false;
+  static const bool fp4_on = [] { const char* v = getenv("APNN_FP4"); return !(v && v[0] == '0'); }();
+  if (!fp4_on || tc5_gemm_planes_clocks(wbits, xbits, M, N, K) == 0) return false;
   const int sms = device_sm_count();
   const PlanesPlan pl = plan_planes(wbits, xbits, M, N, K, sms);
   const long long tiles = (((long long)M + pl.np - 1) / pl.np) * ((N + HALF - 1) / HALF);

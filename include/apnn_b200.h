@@ -57,8 +57,9 @@ enum { APNN_SIGN_NONE = 0, APNN_SIGN_W = 1, APNN_SIGN_X = 2 };
 enum { APNN_POOL_NONE = 0, APNN_POOL_AVG2 = 1, APNN_POOL_MAX2 = 2 };
 /* Contraction path. */
 enum {
-  APNN_ALGO_AUTO = 0,    /* TCGEN05 when a large enough workspace is given and the problem is
-                            big enough to fill the device, else IMMA */
+  APNN_ALGO_AUTO = 0,    /* with a large enough workspace: the one-launch kernel of apnn_gemm_planes
+                            for 1- and 2-bit operands in one wave of tiles, TCGEN05 for problems
+                            big enough to fill the device; else IMMA */
   APNN_ALGO_BMMA = 1,    /* 1-bit and-popcount mma.sync per plane pair (emulated on sm_100a;
                             kept as the measured comparison), no workspace */
   APNN_ALGO_IMMA = 2,    /* planes spread to u8 in registers, mma.sync m16n8k32, no workspace */
