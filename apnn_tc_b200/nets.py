@@ -617,20 +617,22 @@ class Network:
         return self._launch_conv(ls, sh, X, a, B, epi, out, s)
 
     def _launch_conv(self, ls, sh, X, a, B, epi, out, s) -> int:
+        # every int8 form, the first layer's too, may be the producer in front of layers on e2m1 operands only
+        conv_i8 = self.L.apnn_conv2d_i8_to_fp4 if epi.out_i8 == _cabi.ROWS_FP4 else self.L.apnn_conv2d_i8
         if self.first_blocks and self.first_blocks[0] == ls.name:
             _, Hb, Wb, bh, taps = self.first_blocks
             epi.in_halo = bh
             # filter bytes -1 / 0 / +1 (bit 0), centred signed image bytes (bit 1)
-            _cabi.check(self.L.apnn_conv2d_i8(s, self.w8[ls.name].data_ptr(), self.xblocks.data_ptr(), out.data_ptr(), B,
-                                              Hb, Wb, 64, sh["coutp"], taps, 1, 3, ctypes.byref(epi), self.flag.data_ptr()),
+            _cabi.check(conv_i8(s, self.w8[ls.name].data_ptr(), self.xblocks.data_ptr(), out.data_ptr(), B,
+                                Hb, Wb, 64, sh["coutp"], taps, 1, 3, ctypes.byref(epi), self.flag.data_ptr()),
                         "apnn_conv2d_i8 " + ls.name)
             return 1
         if self.first_im2col and self.first_im2col[0] == ls.name:
             _, Hc, Wc, kp = self.first_im2col
             epi.in_halo = 0
             signs = 3 if self.spec.first_bits == 8 else 1   # bit 0: -1/+1 filter bytes; bit 1: centred (signed) image bytes
-            _cabi.check(self.L.apnn_conv2d_i8(s, self.w8[ls.name].data_ptr(), self.x8.data_ptr(), out.data_ptr(), B,
-                                              Hc, Wc, kp, sh["coutp"], 1, 1, signs, ctypes.byref(epi), self.flag.data_ptr()),
+            _cabi.check(conv_i8(s, self.w8[ls.name].data_ptr(), self.x8.data_ptr(), out.data_ptr(), B,
+                                Hc, Wc, kp, sh["coutp"], 1, 1, signs, ctypes.byref(epi), self.flag.data_ptr()),
                         "apnn_conv2d_i8 " + ls.name)
             return 1
         if self.fp4.get(ls.name, False):
@@ -644,10 +646,9 @@ class Network:
                 rows = X.shape[1] * X.shape[2] * X.shape[3]
                 _cabi.check(self.L.apnn_expand_planes(s, X.data_ptr(), self.x8.data_ptr(), rows, sh["cinp"], a, 0), "expand")
                 n, x8 = 2, self.x8
-            conv = self.L.apnn_conv2d_i8_to_fp4 if epi.out_i8 == _cabi.ROWS_FP4 else self.L.apnn_conv2d_i8
-            _cabi.check(conv(s, self.w8[ls.name].data_ptr(), x8.data_ptr(), out.data_ptr(), B,
-                             sh["H"], sh["W"], sh["cinp"], sh["coutp"], ls.R, ls.stride, 1,
-                             ctypes.byref(epi), self.flag.data_ptr()), "apnn_conv2d_i8 " + ls.name)
+            _cabi.check(conv_i8(s, self.w8[ls.name].data_ptr(), x8.data_ptr(), out.data_ptr(), B,
+                                sh["H"], sh["W"], sh["cinp"], sh["coutp"], ls.R, ls.stride, 1,
+                                ctypes.byref(epi), self.flag.data_ptr()), "apnn_conv2d_i8 " + ls.name)
             return n
         epi.signed_operand = _cabi.SIGN_W
         _cabi.check(self.L.apnn_conv2d_ex(s, _cabi.ALGO_IMMA, 1, a, self.w_planes[ls.name].data_ptr(), X.data_ptr(),

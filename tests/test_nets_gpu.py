@@ -115,3 +115,42 @@ def test_graph_replay_matches_eager(cuda_device):
     replayed = net.replay().clone()
     net.check()
     assert torch.equal(replayed, second) and not torch.equal(eager, second)
+
+
+def _small_spec(name, hw, first_bits, *layers):
+    from apnn_tc_b200 import nets
+    return nets.ModelSpec(name, hw, 3, list(layers), first_bits=first_bits)
+
+
+def _first_layer_specs():
+    """Unpooled first convolutions whose only consumers run on e2m1 operands, so that they write nibble rows themselves:
+    pixel blocks with 3x3 and 5x5 block taps, gathered windows, a fully connected and a convolutional consumer, a saved
+    residual beside the rows."""
+    from apnn_tc_b200.nets import LayerSpec as L
+    fc, out = L("Fc1", "fc", 0, 256), L("Fout", "out", 256, 100, quantise=False)
+    wide = L("Conv2", "conv", 128, 256, 3)
+    for bits in (8, 0):
+        yield _small_spec(f"blocks3_fc_{bits}", 32, bits, L("Conv1", "conv", 3, 64, 7, 4), fc, out)
+        yield _small_spec(f"blocks5_fc_{bits}", 32, bits, L("Conv1", "conv", 3, 64, 11, 4), fc, out)
+        yield _small_spec(f"gathered_fc_{bits}", 16, bits, L("Conv1", "conv", 3, 64, 3, 2), fc, out)
+        yield _small_spec(f"blocks3_conv_{bits}", 48, bits, L("Conv1", "conv", 3, 128, 7, 4), wide, fc, out)
+        yield _small_spec(f"gathered_conv_{bits}", 12, bits, L("Conv1", "conv", 3, 128, 3, save_residual=True), wide, fc, out)
+
+
+@pytest.mark.parametrize("index", range(10))
+def test_unpooled_first_layer_feeds_e2m1_layers(cuda_device, index):
+    from apnn_tc_b200 import nets
+    spec = list(_first_layer_specs())[index]
+    params = nets.make_params(spec, narrow=True)
+    images = np.random.default_rng(index).uniform(-10, 10, size=(3, spec.image_hw, spec.image_hw, 3)).astype(np.float32)
+    want, levels, values = forward_reference(spec, params, images)
+    net = nets.Network(spec, 3, params)
+    assert net.fp4_out["Conv1"]
+    logits = net.forward(torch.from_numpy(images).cuda())
+    net.check()
+    for name in levels:
+        if name is not None and name.startswith("Conv"):
+            assert np.array_equal(net.levels_of(name).cpu().numpy(), levels[name]), name
+    for name in net.res:
+        assert np.array_equal(net.res[name].cpu().numpy().astype(np.int32).reshape(values[name].shape), values[name])
+    assert np.array_equal(logits.cpu().numpy(), want) and len(np.unique(levels["Conv1"])) > 1
