@@ -482,7 +482,6 @@ tc5_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const int lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    if (blockIdx.x == 0) *p.error_flag = 0;  // only ever raised after a 2 s wait, long after this store
     for (int s = 0; s < stages; s++) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -537,6 +536,9 @@ tc5_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     // ---------------- TMA producer ----------------
     if (lane == 0) {
       grid_dependency_wait();   // the first load of anything an earlier kernel wrote comes after this
+      // behind the wait like every other store: the flag may lie in memory that the previous kernel still reads or writes.
+      // (Other roles raise it after a 2 s wait at the earliest, long after this store.)
+      if (blockIdx.x == 0) *p.error_flag = 0;
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;

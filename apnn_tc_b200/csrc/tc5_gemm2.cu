@@ -227,6 +227,7 @@ tc5_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   const uint32_t bars = base + (MX ? (uint32_t)p.stages * MX_STAGE_BYTES : STAGES * STAGE_BYTES);
   const uint32_t epi_bytes = (MX && p.stages == MX_DEEP_STAGES) ? MX_DEEP_EPI_BYTES : THR_BYTES_PER_WARP;
   if (MX && (raw & 1023u) != 0) {   // never seen; the swizzled tiles and the bulk stores need the alignment
+    grid_dependency_wait();
     if (threadIdx.x == 0) atomicExch(p.error_flag, 9);
     return;
   }
