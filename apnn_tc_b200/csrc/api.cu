@@ -248,8 +248,9 @@ apnn_status apnn_gemm_ex(void* stream, int algo, int wbits, int xbits, const voi
     // the expand pass and the tcgen05 kernels: many tiles, or two gigaoperations that are not a skinny problem, whose wide
     // operand the expand pass would write and read for few uses (int32, us: 2048 x 2048 x 256 8.3 against 12.2 on the
     // warp-level kernel, packed output 11.5 / 27.2; 8192 x 512 x 512 9.3 / 12.1; but 64 x 4096 x 4096 14.3 / 9.5)
-    const bool big = tc5_worthwhile(M, N, K) || (M >= 512 && N >= 512 && 2.0 * M * N * K >= 2e9);
-    algo = (ws_ok && (big || !warp_ok)) ? APNN_ALGO_TCGEN05 : APNN_ALGO_IMMA;
+    // (The second kind also has a warp-level kernel, which takes a workspace of any alignment.)
+    const bool mid = aligned32(workspace) && M >= 512 && N >= 512 && 2.0 * M * N * K >= 2e9;
+    algo = (ws_ok && (tc5_worthwhile(M, N, K) || mid || !warp_ok)) ? APNN_ALGO_TCGEN05 : APNN_ALGO_IMMA;
   }
   if (!warp_ok && algo != APNN_ALGO_TCGEN05 && algo != APNN_ALGO_TCGEN05_PAIR)
     return workspace ? APNN_ERR_UNSUPPORTED : APNN_ERR_WORKSPACE;

@@ -5,6 +5,7 @@ import os
 import re
 
 import pytest
+import torch
 
 from apnn_tc_b200 import _cabi
 
@@ -87,6 +88,20 @@ def test_argument_validation_returns_status_codes():
     # packers
     assert L.apnn_bit_compress(None, p, p, 0, 3, 2) == 1
     assert L.apnn_quantize_pack(None, p, p, 4, 3, 9) == 1
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host addresses stand in for device memory: only without a device")
+def test_automatic_choice_takes_workspaces_of_any_alignment():
+    """A problem the warp-level kernel takes is not refused for where its workspace lies.  Without a device an accepted call
+    ends in the CUDA error of its first launch (5), a refused one in its own status."""
+    L = _cabi.lib()
+    buf = (ctypes.c_uint32 * 64)()
+    base = ctypes.addressof(buf)
+    p = base + (-base % 32)
+    for wbits, xbits, M, N, K in ((1, 2, 512, 2048, 1024), (2, 2, 1024, 1024, 1024), (1, 4, 600, 700, 2560), (1, 2, 64, 128, 128)):
+        size = L.apnn_gemm_workspace_bytes(3, wbits, xbits, M, N, K)
+        for offset in (0, 16, 4):
+            assert L.apnn_gemm_ex(None, 0, wbits, xbits, p, p, p, M, N, K, None, p + offset, size) == 5, (M, N, K, offset)
 
 
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
