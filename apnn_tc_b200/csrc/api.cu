@@ -105,6 +105,15 @@ int pdl_attribute(cudaLaunchAttribute* attrs) {
   return 1;
 }
 
+// The warp-level kernels have no waits to report on: they leave the flag of the caller's workspace at 0.  The kernel stores
+// it (a 4-byte memset in front of the launch took 3 us of an 11 us call at M = 64), unless the slot is not an int's address:
+// these kernels need nothing else of a workspace, so one at any address is accepted.
+static cudaError_t clear_status_flag(CoreParams& p, int* slot, cudaStream_t s) {
+  if ((reinterpret_cast<uintptr_t>(slot) & 3u) != 0) return cudaMemsetAsync(slot, 0, sizeof(int), s);
+  p.clear_flag = slot;
+  return cudaSuccess;
+}
+
 // Plane counts the int8 (tcgen05) path takes: every level of up to 8 bits fits one byte.
 bool tc5_bits_ok(int bits) { return (bits >= 1 && bits <= 4) || bits == 8; }
 
@@ -240,8 +249,9 @@ apnn_status apnn_gemm_ex(void* stream, int algo, int wbits, int xbits, const voi
 
   if (algo == APNN_ALGO_AUTO) {
     const bool ws_ok = workspace && workspace_bytes >= tc5_workspace_bytes(M, N, K);
-    // operands of at most two bits, one wave of tiles: straight from the planes in one launch
-    if (ws_ok && !(epi && epi->n_peer_out != 0) &&
+    // operands of at most two bits, one wave of tiles: straight from the planes in one launch (of the workspace it only uses
+    // the status flag, which has to be an int's address)
+    if (ws_ok && (reinterpret_cast<uintptr_t>(workspace) & 3u) == 0 && !(epi && epi->n_peer_out != 0) &&
         tc5_gemm_planes_preferred(wbits, xbits, M, N, K, epi && epi->out_mode != APNN_OUT_INT32))
       return tc5_gemm_planes(s, wbits, xbits, (const uint32_t*)W, (const uint32_t*)X, D, M, N, K, epi,
                              tc5_flag_slot(workspace, M, N, K));
@@ -266,9 +276,10 @@ apnn_status apnn_gemm_ex(void* stream, int algo, int wbits, int xbits, const voi
   memset(&p, 0, sizeof(p));
   p.A = (const uint32_t*)W;
   p.B = (const uint32_t*)X;
-  // the warp-level kernels have no waits; the flag apnn_gemm_check reads is cleared by the kernel itself (as a memset of
-  // its own in front of the launch it took 3 us of an 11 us call at M = 64)
-  if (workspace && workspace_bytes >= tc5_workspace_bytes(M, N, K)) p.clear_flag = tc5_flag_slot(workspace, M, N, K);
+  if (workspace && workspace_bytes >= tc5_workspace_bytes(M, N, K)) {
+    cudaError_t ce = clear_status_flag(p, tc5_flag_slot(workspace, M, N, K), s);
+    if (ce != cudaSuccess) return cuda_fail(ce, "status flag reset");
+  }
   p.a_plane_words = (long long)M * (K / 32);
   p.b_plane_words = (long long)N * (K / 32);
   p.M = M;
@@ -447,8 +458,11 @@ apnn_status apnn_conv2d_ex(void* stream, int algo, int wbits, int xbits, const v
   memset(&p, 0, sizeof(p));
   p.A = (const uint32_t*)X;
   p.B = (const uint32_t*)Wt;
-  if (workspace && workspace_bytes >= tc5_conv_workspace_bytes(B, H, Wd, CIN, COUT, R))
-    p.clear_flag = tc5_conv_flag_slot(workspace, B, H, Wd, CIN, COUT, R);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (workspace && workspace_bytes >= tc5_conv_workspace_bytes(B, H, Wd, CIN, COUT, R)) {
+    cudaError_t ce = clear_status_flag(p, tc5_conv_flag_slot(workspace, B, H, Wd, CIN, COUT, R), s);
+    if (ce != cudaSuccess) return cuda_fail(ce, "status flag reset");
+  }
   const int in_halo = (epi && epi->in_halo) ? epi->in_halo : pad;
   if (in_halo < pad) return APNN_ERR_INVALID_ARG;
   p.Hp = H + 2 * in_halo;
@@ -484,7 +498,6 @@ apnn_status apnn_conv2d_ex(void* stream, int algo, int wbits, int xbits, const v
   }
   p.out_plane_words =
       (long long)B * (p.out_h + 2 * p.out_halo) * (p.out_w + 2 * p.out_halo) * (COUT / 32);
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   cudaError_t e = launch_core(CORE_U8, xbits, wbits, p, s, core_pick_tile(p, device_sm_count()));
   if (e != cudaSuccess) return cuda_fail(e, "apnn_conv2d launch");
   return APNN_OK;

@@ -104,6 +104,28 @@ def test_automatic_choice_takes_workspaces_of_any_alignment():
             assert L.apnn_gemm_ex(None, 0, wbits, xbits, p, p, p, M, N, K, None, p + offset, size) == 5, (M, N, K, offset)
 
 
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host addresses stand in for device memory: only without a device")
+def test_status_flag_of_an_unaligned_workspace_is_not_stored_by_a_kernel():
+    """A kernel stores the status flag only at a 4-byte-aligned address; elsewhere it is a memset, which is then the call that
+    finds no device."""
+    L = _cabi.lib()
+    buf = (ctypes.c_uint32 * 64)()
+    base = ctypes.addressof(buf)
+    p = base + (-base % 32)
+    e = _cabi.Epilogue(out_mode=1, out_bits=2)
+    for offset in (0, 1, 2, 3, 4, 6, 16, 17):
+        reset = offset % 4 != 0
+        for algo in (0, 1, 2):
+            for M, N, K, epi in ((64, 128, 128, None), (64, 128, 128, e), (128, 4096, 9216, e), (512, 2048, 1024, None)):
+                size = L.apnn_gemm_workspace_bytes(3, 1, 2, M, N, K)
+                assert L.apnn_gemm_ex(None, algo, 1, 2, p, p, p, M, N, K, None if epi is None else ctypes.byref(epi), p + offset, size) == 5
+                assert L.apnn_last_cuda_error().startswith(b"status flag reset") == reset, (algo, M, N, K, offset)
+            if algo != 1:
+                size = L.apnn_conv2d_workspace_bytes(3, 1, 8, 8, 128, 64, 3)
+                assert L.apnn_conv2d_ex(None, algo, 1, 2, p, p, p, 1, 8, 8, 128, 64, 3, 1, None, p + offset, size) == 5
+                assert L.apnn_last_cuda_error().startswith(b"status flag reset") == reset, (algo, offset)
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_cabi, "_lib", None)
     monkeypatch.setattr(_cabi, "LIB_PATH", str(tmp_path / "nope.so"))

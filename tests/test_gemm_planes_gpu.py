@@ -65,3 +65,25 @@ def test_planes_gemm_residuals_and_large_thresholds(cuda_device):
     out = torch.zeros((2, M, N // 32), dtype=torch.int32, device="cuda")
     assert np.array_equal(to_host(run(to_dev(W), to_dev(X), out, epi, 1, 2, M, N, K)), oracle.requant_pack(v, 2, 2, T))
     assert np.array_equal(rout.cpu().numpy(), v)
+
+
+@pytest.mark.parametrize("offset", [0, 4, 16, 1, 18])
+@pytest.mark.parametrize("M,N,K,mode", [(64, 128, 128, "int32"), (64, 128, 128, "lowbits"), (1024, 1024, 1024, "int32")])
+def test_automatic_choice_with_a_workspace_at_any_offset(cuda_device, offset, M, N, K, mode):
+    """The status flag is left at 0 wherever the workspace lies, by the kernel or, at an odd address, by a memset."""
+    import apnn_tc_b200 as ap
+    from apnn_tc_b200 import _cabi
+    from apnn_tc_b200.ops import _stream_ptr
+    rng = np.random.default_rng(offset + M)
+    W, _ = oracle.value_planes(rng, M, K, 1)
+    X, _ = oracle.value_planes(rng, N, K, 2)
+    v = oracle.gemm_popc(W, X, threads=8)
+    size = ap.gemm_workspace_bytes(M, N, K)
+    ws = torch.full((size + 32,), 0xEE, dtype=torch.uint8, device="cuda")[offset:offset + size]
+    epi = ap.make_epilogue(mode, 2) if mode != "int32" else None
+    got = ap.apmm(to_dev(W), to_dev(X), workspace=ws, epilogue=epi)
+    _cabi.check(_cabi.lib().apnn_gemm_check(_stream_ptr(), ws.data_ptr(), M, N, K))
+    if mode == "int32":
+        assert np.array_equal(to_host(got, np.int32), v)
+    else:
+        assert np.array_equal(to_host(got), oracle.requant_pack(v, 2, 1, None))
