@@ -502,7 +502,9 @@ class Network:
             self.image_levels = torch.zeros((a, B, self.hw, self.hw, cp // 32), dtype=torch.int32,
                                             device=self.device) if h0 else None
         self.x8 = torch.empty(max(x8_bytes, 256), dtype=torch.uint8, device=self.device)
-        self.flag = torch.zeros(1, dtype=torch.int32, device=self.device)
+        # one status word per layer: every kernel clears its own before it starts, so a shared one would only tell of the last
+        self.flag = torch.zeros(len(spec.layers), dtype=torch.int32, device=self.device)
+        self._slot = {ls.name: i for i, ls in enumerate(spec.layers)}
         self.graph = None
         self.static_images = None
         self.launches_per_forward = 0
@@ -578,6 +580,9 @@ class Network:
             return None if self.first_im2col else self.image_planes   # the im2col first layer reads self.x8
         return self.out[src]
 
+    def _flag_of(self, ls: LayerSpec) -> int:
+        return self.flag.data_ptr() + 4 * self._slot[ls.name]
+
     def _epilogue(self, ls: LayerSpec, conv: bool):
         if ls.name in self.affine:
             sc, bi = self.affine[ls.name]
@@ -624,7 +629,7 @@ class Network:
             epi.in_halo = bh
             # filter bytes -1 / 0 / +1 (bit 0), centred signed image bytes (bit 1)
             _cabi.check(conv_i8(s, self.w8[ls.name].data_ptr(), self.xblocks.data_ptr(), out.data_ptr(), B,
-                                Hb, Wb, 64, sh["coutp"], taps, 1, 3, ctypes.byref(epi), self.flag.data_ptr()),
+                                Hb, Wb, 64, sh["coutp"], taps, 1, 3, ctypes.byref(epi), self._flag_of(ls)),
                         "apnn_conv2d_i8 " + ls.name)
             return 1
         if self.first_im2col and self.first_im2col[0] == ls.name:
@@ -632,13 +637,13 @@ class Network:
             epi.in_halo = 0
             signs = 3 if self.spec.first_bits == 8 else 1   # bit 0: -1/+1 filter bytes; bit 1: centred (signed) image bytes
             _cabi.check(conv_i8(s, self.w8[ls.name].data_ptr(), self.x8.data_ptr(), out.data_ptr(), B,
-                                Hc, Wc, kp, sh["coutp"], 1, 1, signs, ctypes.byref(epi), self.flag.data_ptr()),
+                                Hc, Wc, kp, sh["coutp"], 1, 1, signs, ctypes.byref(epi), self._flag_of(ls)),
                         "apnn_conv2d_i8 " + ls.name)
             return 1
         if self.fp4.get(ls.name, False):
             _cabi.check(self.L.apnn_conv2d_fp4(s, self.w4[ls.name].data_ptr(), X.data_ptr(), out.data_ptr(), B, sh["H"],
                                                sh["W"], sh["cinp"], sh["coutp"], ls.R, ctypes.byref(epi),
-                                               self.flag.data_ptr()), "apnn_conv2d_fp4 " + ls.name)
+                                               self._flag_of(ls)), "apnn_conv2d_fp4 " + ls.name)
             return 1
         if self.tc5_ok[ls.name]:
             n, x8 = 1, X
@@ -648,7 +653,7 @@ class Network:
                 n, x8 = 2, self.x8
             _cabi.check(conv_i8(s, self.w8[ls.name].data_ptr(), x8.data_ptr(), out.data_ptr(), B,
                                 sh["H"], sh["W"], sh["cinp"], sh["coutp"], ls.R, ls.stride, 1,
-                                ctypes.byref(epi), self.flag.data_ptr()), "apnn_conv2d_i8 " + ls.name)
+                                ctypes.byref(epi), self._flag_of(ls)), "apnn_conv2d_i8 " + ls.name)
             return n
         epi.signed_operand = _cabi.SIGN_W
         _cabi.check(self.L.apnn_conv2d_ex(s, _cabi.ALGO_IMMA, 1, a, self.w_planes[ls.name].data_ptr(), X.data_ptr(),
@@ -665,7 +670,7 @@ class Network:
         s = _stream_ptr()
         if self.fp4.get(ls.name, False):
             _cabi.check(self.L.apnn_linear_fp4(s, X.data_ptr(), self.w4[ls.name].data_ptr(), out.data_ptr(), B, N, K,
-                                               ctypes.byref(epi), self.flag.data_ptr()), "apnn_linear_fp4 " + ls.name)
+                                               ctypes.byref(epi), self._flag_of(ls)), "apnn_linear_fp4 " + ls.name)
             return 1
         if self.tc5_ok[ls.name]:
             n, x8 = 1, X
@@ -673,7 +678,7 @@ class Network:
                 _cabi.check(self.L.apnn_expand_planes(s, X.data_ptr(), self.x8.data_ptr(), B, K, a, 0), "expand")
                 n, x8 = 2, self.x8
             _cabi.check(self.L.apnn_gemm_i8(s, x8.data_ptr(), self.w8[ls.name].data_ptr(), out.data_ptr(), B, N, K,
-                                            0, 1, ctypes.byref(epi), self.flag.data_ptr()), "apnn_gemm_i8 " + ls.name)
+                                            0, 1, ctypes.byref(epi), self._flag_of(ls)), "apnn_gemm_i8 " + ls.name)
             return n
         if ls.name in self.affine:
             plain = make_epilogue("int32", signed="x")
@@ -767,7 +772,8 @@ class Network:
         return self.out[self.spec.layers[-1].name]
 
     def check(self) -> None:
-        """Synchronise and raise if a tcgen05 kernel gave up on a bounded wait."""
+        """Synchronise and raise if a tcgen05 kernel of the last forward pass gave up on a bounded wait."""
         torch.cuda.synchronize(self.device)
-        if int(self.flag.item()) != 0:
-            raise _cabi.ApnnError(7, "a bounded device-side wait expired")
+        gave_up = [ls.name for ls, f in zip(self.spec.layers, self.flag.tolist()) if f]
+        if gave_up:
+            raise _cabi.ApnnError(7, "a bounded device-side wait expired in " + ", ".join(gave_up))

@@ -154,3 +154,26 @@ def test_unpooled_first_layer_feeds_e2m1_layers(cuda_device, index):
     for name in net.res:
         assert np.array_equal(net.res[name].cpu().numpy().astype(np.int32).reshape(values[name].shape), values[name])
     assert np.array_equal(logits.cpu().numpy(), want) and len(np.unique(levels["Conv1"])) > 1
+
+
+@pytest.mark.parametrize("model,name", [("resnet18", "L1B1C1"), ("alexnet", "Conv4"), ("alexnet", "Fc1"), ("vgg_variant", "Fout")])
+def test_check_reports_a_layer_that_gave_up(cuda_device, model, name):
+    """A status raised by one layer is still there after the layers behind it have run.  (Written from the host where the
+    layer's kernel would have written it.)"""
+    from apnn_tc_b200 import _cabi, nets
+    from apnn_tc_b200.ops import _stream_ptr
+    spec = nets.MODELS[model](n_classes=100)
+    net = nets.Network(spec, 2, image_hw=64)
+    images = torch.rand((2, 64, 64, 3), device="cuda") * 20 - 10
+    net.forward(images)
+    net.check()
+    contractions = [i for i, call in enumerate(net._calls) if call[2] not in ("apnn_maxpool2x2_rows", "apnn_expand_planes")][1:]
+    at = contractions[[ls.name for ls in spec.layers].index(name)]
+    address = net._calls[at][1][-1].value
+    net.flag[(address - net.flag.data_ptr()) // 4] = 3
+    for fn, args, what in net._calls[at + 1:]:
+        _cabi.check(fn(_stream_ptr(), *args), what)
+    with pytest.raises(_cabi.ApnnError):
+        net.check()
+    net.forward(images)
+    net.check()
