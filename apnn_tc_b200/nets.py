@@ -328,6 +328,34 @@ class _CallList:
         return collect
 
 
+class _Changes:
+    """Counts what has been exchanged in a network since its construction."""
+
+    def __init__(self):
+        self.count = 0
+
+
+class _Entries(dict):
+    """A dict of a network's buffers or plans that counts every exchange of an entry."""
+
+    def __init__(self, entries, changes: _Changes):
+        super().__init__(entries)
+        self._changes = changes
+
+
+def _counted(name):
+    method = getattr(dict, name)
+
+    def change(self, *args, **kw):
+        self._changes.count += 1
+        return method(self, *args, **kw)
+    return change
+
+
+for _name in ("__setitem__", "__delitem__", "__ior__", "clear", "pop", "popitem", "setdefault", "update"):
+    setattr(_Entries, _name, _counted(_name))
+
+
 class Network:
     """A model list bound to device buffers: weights (packed planes, and their int8 images for the
     tcgen05 path, expanded once), one output buffer per layer (packed planes inside the zero ring
@@ -336,7 +364,23 @@ class Network:
     ``forward(images)`` launches one packer and then, per layer, at most an activation expand and
     one contraction kernel, all on the current stream; ``capture()`` records that sequence in a
     CUDA graph for replay.
+
+    The buffers may be written in place at any time, and entries of ``thr``, ``out``, ``res``, ``flag`` and the other
+    members exchanged: the next ``forward()`` uses the new tensors (a graph keeps those it was captured with).  Exchanging
+    the storage inside a tensor (``t.data = ...``) goes unnoticed; assign the tensor again after it.  The weights of a layer
+    on e2m1 operands are in ``w4``, those of the other tcgen05 layers in ``w8``.
     """
+
+    # members that forward()'s calls do not depend on
+    _PASSIVE = frozenset(("L", "graph", "static_images", "launches_per_forward", "_calls", "_calls_at"))
+
+    def __setattr__(self, name, value):
+        if name not in self._PASSIVE:
+            changes = self.__dict__.setdefault("_changes", _Changes())
+            changes.count += 1
+            if type(value) is dict:
+                value = _Entries(value, changes)
+        object.__setattr__(self, name, value)
 
     def __init__(self, spec: ModelSpec, batch: int, params: Optional[Dict[str, LayerParams]] = None,
                  device: Optional[torch.device] = None, image_hw: Optional[int] = None, use_tcgen05: bool = True):
@@ -508,8 +552,9 @@ class Network:
         self.graph = None
         self.static_images = None
         self.launches_per_forward = 0
-        # forward()'s calls in order; None where it also copies with torch (the packed first layer) and issues them one by one
-        self._calls = None if self.first_im2col is None else self._lay_out()
+        self._calls = self._calls_at = None   # forward()'s calls in order, and the count of changes they were laid out at
+        if self.first_im2col is not None:
+            self._lay_out()
         torch.cuda.synchronize(self.device)
 
     def _fp4_candidate(self, ls: LayerSpec) -> bool:
@@ -727,25 +772,27 @@ class Network:
             n += self._run_conv(ls) if ls.kind == "conv" else self._run_fc(ls)
         self.launches_per_forward = n
 
-    def _lay_out(self) -> list:
+    def _lay_out(self) -> None:
         lib, record = self.L, _CallList(self.L)
         try:
             self.L = record
             self._issue(self.flag)    # stands in for the images, whose address the first call takes at run time
         finally:
             self.L = lib
-        return record.calls
+        self._calls, self._calls_at = record.calls, self._changes.count
 
     def forward(self, images: torch.Tensor) -> torch.Tensor:
         """images: float32 [B, H, W, C] on the device.  Returns the logits [B, PAD128(classes)]: float32 with
         ``float_logits`` (the default), else the int32 values.
 
-        Issues the sequence of C calls laid out at construction (arguments are the network's own buffers, the stream and
-        the image address excepted).  Building every descriptor anew took the host 10 us per layer, more than the GPU
-        needs at a small batch: ResNet-18 at 8 images 232 -> 218 us."""
-        if self._calls is None:
+        Issues the sequence of C calls laid out at construction, or since the last exchange of a buffer (arguments are the
+        network's own buffers, the stream and the image address excepted).  Building every descriptor anew took the host
+        10 us per layer, more than the GPU needs at a small batch: ResNet-18 at 8 images 232 -> 218 us."""
+        if self.first_im2col is None:   # the packed first layer is also copied with torch: issued call by call
             self._issue(images)
             return self.out[self.spec.layers[-1].name]
+        if self._calls_at != self._changes.count:
+            self._lay_out()
         s, image = _stream_ptr(), images.data_ptr()
         for i, (fn, args, name) in enumerate(self._calls):
             st = fn(s, image, *args[1:]) if i == 0 else fn(s, *args)   # the first call alone reads the images

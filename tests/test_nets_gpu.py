@@ -177,3 +177,32 @@ def test_check_reports_a_layer_that_gave_up(cuda_device, model, name):
         net.check()
     net.forward(images)
     net.check()
+
+
+@pytest.mark.parametrize("model", ["resnet18", "alexnet", "vgg_variant"])
+def test_exchanged_buffers_take_effect(cuda_device, model):
+    """Entries of a network's buffers replaced after construction are what the next forward pass uses."""
+    from apnn_tc_b200 import nets
+    spec = nets.MODELS[model](n_classes=100)
+    params = nets.make_params(spec, image_hw=64)
+    images = torch.rand((2, 64, 64, 3), device="cuda") * 20 - 10
+    net = nets.Network(spec, 2, params, image_hw=64)
+    first = net.forward(images).clone()
+    hidden = [ls.name for ls in spec.layers if ls.quantise and net.thr[ls.name] is not None]
+    for name in hidden[1:3]:
+        params[name].thresholds = np.where(params[name].thresholds == 2**31 - 1, 2**31 - 1, params[name].thresholds + 7).astype(np.int32)
+        net.thr[name] = torch.from_numpy(params[name].thresholds).cuda()
+    want = nets.Network(spec, 2, params, image_hw=64).forward(images)
+    assert not torch.equal(want, first)
+    assert torch.equal(net.forward(images), want)
+    kept = {name: t for name, t in list(net.out.items()) + list(net.res.items())}
+    for d in (net.out, net.res, net.w8, net.w4):
+        d.update({name: t.clone() for name, t in d.items()})
+    net.flag, net.unpooled = torch.full_like(net.flag, 9), net.unpooled.clone()
+    for t in kept.values():
+        t.fill_(77)
+    assert torch.equal(net.forward(images), want)
+    assert all(bool((t == 77).all()) for t in kept.values())      # nothing wrote the old tensors
+    net.check()
+    net.capture(images)
+    assert torch.equal(net.replay(), want)
