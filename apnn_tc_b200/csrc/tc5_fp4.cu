@@ -378,6 +378,7 @@ struct Fp4Plan {
   int np;          // 0: not applicable
   int splits;      // pairs of a cluster that share a tile's K
   long long clk;   // estimated SM clocks
+  long long waves; // tiles of a pair
 };
 int fp4_cluster_capacity(int splits, int span);
 
@@ -386,12 +387,12 @@ int fp4_cluster_capacity(int splits, int span);
 // epilogue chunks), the pixel box at most 256 rows; a split problem is one wave of resident clusters, and is taken when it
 // saves a tenth.
 Fp4Plan plan_np(long long flat_rows, int COUT, int R, int Wp, int kbytes_per_tap, int span, int sms) {
-  Fp4Plan best = {0, 1, 0};
+  Fp4Plan best = {0, 1, 0, 0};
   const long long cblocks = kbytes_per_tap / span;
   const long long tiles_n = (COUT + TILE_CH - 1) / TILE_CH;
   const int pairs = sms / 2;
   for (int splits = 1; splits <= 4 && splits * 2 <= cblocks + (splits == 1 ? 1 : 0); splits *= 2) {
-    Fp4Plan here = {0, splits, 0};
+    Fp4Plan here = {0, splits, 0, 0};
     for (int np = MAX_NP; np >= 32; np -= 32) {
       const int rows = box_rows_of(R, Wp, np);
       if (rows > 256) continue;
@@ -408,7 +409,7 @@ Fp4Plan plan_np(long long flat_rows, int COUT, int R, int Wp, int kbytes_per_tap
         if (per < stream) per = stream;
       }
       const long long clk = waves * (per > epi ? per : epi) + epi / splits + 6000 + (splits > 1 ? 2000 : 0);
-      if (here.np == 0 || clk < here.clk) here = {np, splits, clk};
+      if (here.np == 0 || clk < here.clk) here = {np, splits, clk, waves};
     }
     if (here.np && (best.np == 0 || here.clk * 10 <= best.clk * 9)) best = here;
   }
@@ -512,15 +513,41 @@ cudaError_t launch_kind(cudaStream_t s, const CUtensorMap& map_x, const CUtensor
 
 }  // namespace
 
+static bool fp4_takes(int B, int Hin, int Win, int CIN, int R, int in_halo, int out_halo) {
+  if (CIN % 128 != 0 || (R != 1 && R != 3) || (long long)R * R * CIN * 9 >= (1ll << 24)) return false;
+  const long long flat_rows = (long long)B * (Hin + 2 * in_halo) * (Win + 2 * in_halo);
+  const long long out_rows = (long long)B * (Hin + 2 * out_halo) * (Win + 2 * out_halo);
+  return flat_rows < 0x7fffff00LL && out_rows < 0x7fffff00LL;
+}
+
 // Shapes tc5_conv_fp4 takes, and its cost estimate in SM clocks (0: not taken).
 long long tc5_conv_fp4_clocks(int B, int Hin, int Win, int CIN, int COUT, int R, int in_halo, int out_halo) {
-  if (CIN % 128 != 0 || (R != 1 && R != 3) || (long long)R * R * CIN * 9 >= (1ll << 24)) return 0;
+  if (!fp4_takes(B, Hin, Win, CIN, R, in_halo, out_halo)) return 0;
+  const int Hp = Hin + 2 * in_halo, Wp = Win + 2 * in_halo;
+  const Fp4Plan pl = plan_np((long long)B * Hp * Wp, COUT, R, Wp, CIN / 2, CIN % 256 == 0 ? 128 : 64, device_sm_count());
+  return pl.np ? pl.clk : 0;
+}
+
+// Time of the expand pass and tc5_conv_fp4 together, for the choice between this path and int8 (i8_path_us), in us; negative
+// for shapes it does not take.  Fitted to 1826 convolutions (1x1 and 3x3, 128 .. 1024 channels to 96 .. 1024, maps of 4 to
+// 120) and 992 GEMMs timed on both paths, standard deviation 9 %: launches; 0.19 ns per 1000 elements expanded; per
+// tile 0.5 us and its K blocks, whose 64-byte rows (CIN % 256 != 0) arrive at half the rate; the last tile's epilogue, 32
+// pixels of a warp at a time.  thr2: thresholds of at most two bits, no residuals.
+double tc5_conv_fp4_us(int B, int Hin, int Win, int CIN, int COUT, int R, int in_halo, int out_halo, bool thr2) {
+  if (!fp4_takes(B, Hin, Win, CIN, R, in_halo, out_halo)) return -1.0;
   const int Hp = Hin + 2 * in_halo, Wp = Win + 2 * in_halo;
   const long long flat_rows = (long long)B * Hp * Wp;
-  const long long out_rows = (long long)B * (Hin + 2 * out_halo) * (Win + 2 * out_halo);
-  if (flat_rows >= 0x7fffff00LL || out_rows >= 0x7fffff00LL) return 0;
-  const Fp4Plan pl = plan_np(flat_rows, COUT, R, Wp, CIN / 2, CIN % 256 == 0 ? 128 : 64, device_sm_count());
-  return pl.np ? pl.clk : 0;
+  const int span = CIN % 256 == 0 ? 128 : 64;
+  const Fp4Plan pl = plan_np(flat_rows, COUT, R, Wp, CIN / 2, span, device_sm_count());
+  if (pl.np == 0) return -1.0;
+  const double elements = (double)(flat_rows + (long long)COUT * R * R) * CIN;
+  const int kblocks = (CIN / 2 / span + pl.splits - 1) / pl.splits;
+  const double bytes = (double)span * (R * R * HALF + box_rows_of(R, Wp, pl.np));   // operand bytes of a K block
+  const double block_ns = span == 128 ? 362.0 + (R == 1 ? 0.0 : 0.0098 * bytes) : 106.0 + (R == 1 ? 0.0224 : 0.0140) * bytes;
+  const int parts = epi_warps(thr2 ? 1 : 0, span) / 4;
+  const int chunks = (pl.np / 32 + parts - 1) / parts;   // of a warp
+  return 3.3 + 0.19e-6 * elements + pl.waves * (0.53 + 1e-3 * kblocks * block_ns) + chunks * (thr2 ? 1.45 : 2.83) / pl.splits +
+         (pl.splits > 1 ? 3.4 : 0.0);
 }
 
 apnn_status tc5_conv_fp4(cudaStream_t s, const uint8_t* X4, const uint8_t* W4, void* Out, int B, int Hin, int Win, int CIN,

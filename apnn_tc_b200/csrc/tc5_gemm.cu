@@ -1706,6 +1706,78 @@ bool tc5_conv_supported(int H, int W, int R, int stride, int pool) {
   return tc5_conv_box((H - 1) / stride + 1, (W - 1) / stride + 1, pool, &bw, &bh, &bb);
 }
 
+namespace {
+
+// Tiles of an int8 convolution: pixel boxes, or consecutive padded pixels ("flat").
+struct ConvTiling {
+  int bw, bh, bb, tiles_w, tiles_h;   // pixel boxes
+  bool flat;
+  int flat_nblk, flat_blk_rows;
+  TilePlan plan;
+  long long tiles_m;   // tile rows of the formulation taken (pairs of them when plan.pair)
+};
+
+// H, W: output extent; Hp, Wp: stored input extent.
+bool plan_conv(int B, int H, int W, int Hp, int Wp, int CIN, int COUT, int R, int stride, int pool, bool x_signed, int sms,
+               ConvTiling* t) {
+  if (!tc5_conv_box(H, W, pool, &t->bw, &t->bh, &t->bb)) return false;
+  t->tiles_w = (W + t->bw - 1) / t->bw;
+  t->tiles_h = (H + t->bh - 1) / t->bh;
+  const int tiles_m_box = ((B + t->bb - 1) / t->bb) * t->tiles_h * t->tiles_w;
+  const int span = (CIN % 128 == 0) ? 128 : 64;
+  // stride-1 convolutions without pooling run "flat": tiles of 128 consecutive padded pixels,
+  // every tap a row-shifted view of one buffer of consecutive input rows (2-D TMA loads)
+  const long long flat_rows = (long long)B * Hp * Wp;
+  // ... unless that needs more waves of tiles over the SMs than the pixel boxes would (the ring
+  // positions are computed and dropped: tiny images, or a tile count just past a multiple of the
+  // SM count).  Cost of a formulation = waves x tile width.
+  // The pixel-box formulation can also split K over the CTAs of a cluster when it has few tiles.
+  const int kblocks_all = R * R * (CIN / span);
+  // (the flat kernel path does not split K)
+  auto plan_for = [&](long long tiles_m, bool may_split) {
+    return pick_plan(tiles_m, COUT, kblocks_all, sms, pick_bn(tiles_m, COUT, sms), span == 128 && !x_signed, may_split);
+  };
+  const long long flat_tiles_m = (flat_rows + BM - 1) / BM;
+  const TilePlan pl_box = plan_for(tiles_m_box, true), pl_flat = plan_for(flat_tiles_m, false);
+  // (with many waves a few per cent more tiles still win: a flat tile loads 5-8x fewer rows)
+  const long long cost_box = pl_box.cost, cost_flat = pl_flat.cost;
+  const long long many = 8LL * kblocks_all * 256;   // about eight waves of 128-wide tiles
+  t->flat = stride == 1 && pool == APNN_POOL_NONE && flat_rows < 0x7fffff00LL &&
+            (cost_flat <= cost_box || (cost_box >= many && cost_flat * 100 <= cost_box * 105));
+  if (t->flat) {
+    // rows of input one (tile, channel block) needs: one box when it has at most 256 rows (the TMA
+    // limit), else one box per filter row
+    const int all_rows = (BM + (R - 1) * (Wp + 1) + 7) / 8 * 8;
+    t->flat_nblk = all_rows <= 256 ? 1 : R;
+    t->flat_blk_rows = all_rows <= 256 ? all_rows : (BM + R - 1 + 7) / 8 * 8;
+    // the flat plan needs one such buffer plus two filter tiles next to the fixed part; wide
+    // filters on wide images (R >= 9, or R = 7 with 256-column tiles) do not fit and take the pixel boxes
+    const int b_rows_flat = pl_flat.pair ? pl_flat.bn / 2 : pl_flat.bn;
+    const long long need = (long long)TileCfg<64, 64>::FIXED_BYTES + 2LL * b_rows_flat * span +
+                           (long long)t->flat_nblk * t->flat_blk_rows * span;
+    if (need > SMEM_LIMIT) t->flat = false;
+  }
+  t->plan = t->flat ? pl_flat : pl_box;
+  t->tiles_m = t->flat ? flat_tiles_m : tiles_m_box;
+  if (t->plan.pair) t->tiles_m = (t->tiles_m + 1) / 2;
+  return true;
+}
+
+// Time of the expand pass and the int8 kernel together in us, to compare with tc5_conv_fp4_us; fitted to the same
+// timings (standard deviation 9 %).  tiles_m: tile rows (pairs of them when plan.pair); row_ns: per operand row of a K
+// block; base_us: what a convolution's launch takes more than a GEMM's.
+double i8_path_us(const TilePlan& plan, long long tiles_m, int N, int kblocks, double elements, int sms, double row_ns,
+                  double base_us) {
+  const long long units = tiles_m * ((N + plan.bn - 1) / plan.bn) * plan.splits, slots = plan.pair ? sms / 2 : sms;
+  const long long waves = (units + slots - 1) / slots;
+  const int rows = BM + (plan.pair ? plan.bn / 2 : plan.bn);
+  const double loop_ns = ((kblocks + plan.splits - 1) / plan.splits) * (217.0 + rows * row_ns), drain_ns = 2.5 * plan.bn;
+  return base_us + 0.21e-6 * elements + waves * (2.5 + 1e-3 * (loop_ns > drain_ns ? loop_ns : drain_ns)) + 0.0205 * plan.bn +
+         (plan.splits > 1 ? 3.6 : 0.0);
+}
+
+}  // namespace
+
 apnn_status tc5_conv_i8(cudaStream_t s, const uint8_t* X8, const uint8_t* W8, void* Out, int B, int Hin, int Win,
                         int CIN, int COUT, int R, int stride, bool w_signed, const apnn_epilogue* epi,
                         int* status_flag, bool x_signed) {
@@ -1716,19 +1788,19 @@ apnn_status tc5_conv_i8(cudaStream_t s, const uint8_t* X8, const uint8_t* W8, vo
   const int Hp = Hin + 2 * in_halo, Wp = Win + 2 * in_halo;
   const int H = (Hin - 1) / stride + 1, W = (Win - 1) / stride + 1;  // output extent
   const int pool = epi ? epi->pool : APNN_POOL_NONE;
-  int bw = 0, bh = 0, bb = 0;
-  if (!tc5_conv_box(H, W, pool, &bw, &bh, &bb)) return APNN_ERR_UNSUPPORTED;
   cudaError_t e;
   const int sms = device_sm_count();
+  ConvTiling t;
+  if (!plan_conv(B, H, W, Hp, Wp, CIN, COUT, R, stride, pool, x_signed, sms, &t)) return APNN_ERR_UNSUPPORTED;
   Tc5Params p;
   memset(&p, 0, sizeof(p));
-  p.is_conv = 1;
-  p.bw = bw;
-  p.bh = bh;
-  p.bb = bb;
-  p.tiles_w = (W + bw - 1) / bw;
-  p.tiles_h = (H + bh - 1) / bh;
-  p.tiles_m = ((B + bb - 1) / bb) * p.tiles_h * p.tiles_w;
+  p.is_conv = t.flat ? 2 : 1;
+  p.bw = t.bw;
+  p.bh = t.bh;
+  p.bb = t.bb;
+  p.tiles_w = t.tiles_w;
+  p.tiles_h = t.tiles_h;
+  p.tiles_m = (int)t.tiles_m;
   p.Bn = B;
   p.Ho = H;
   p.Wo = W;
@@ -1741,54 +1813,21 @@ apnn_status tc5_conv_i8(cudaStream_t s, const uint8_t* X8, const uint8_t* W8, vo
   p.out_h = pool ? H / 2 : H;
   p.out_w = pool ? W / 2 : W;
   p.out_halo = epi ? epi->out_halo : 0;
-  p.a_box_bytes = (uint32_t)(bw * bh * bb * span);
-  // stride-1 convolutions without pooling run "flat": tiles of 128 consecutive padded pixels,
-  // every tap a row-shifted view of one buffer of consecutive input rows (2-D TMA loads)
+  p.a_box_bytes = (uint32_t)(t.bw * t.bh * t.bb * span);
   const long long flat_rows = (long long)B * Hp * Wp;
-  // ... unless that needs more waves of tiles over the SMs than the pixel boxes would (the ring
-  // positions are computed and dropped: tiny images, or a tile count just past a multiple of the
-  // SM count).  Cost of a formulation = waves x tile width.
-  // The pixel-box formulation can also split K over the CTAs of a cluster when it has few tiles.
-  const int kblocks_all = R * R * p.cblocks;
-  // (the flat kernel path does not split K)
-  auto plan_for = [&](long long tiles_m, bool may_split) {
-    return pick_plan(tiles_m, COUT, kblocks_all, sms, pick_bn(tiles_m, COUT, sms), span == 128 && !x_signed, may_split);
-  };
-  const int tiles_m_box = p.tiles_m;
-  const TilePlan pl_box = plan_for(tiles_m_box, true), pl_flat = plan_for((flat_rows + BM - 1) / BM, false);
-  // (with many waves a few per cent more tiles still win: a flat tile loads 5-8x fewer rows)
-  const long long cost_box = pl_box.cost, cost_flat = pl_flat.cost;
-  const long long many = 8LL * kblocks_all * 256;   // about eight waves of 128-wide tiles
-  bool flat = stride == 1 && pool == APNN_POOL_NONE && flat_rows < 0x7fffff00LL &&
-              (cost_flat <= cost_box || (cost_box >= many && cost_flat * 100 <= cost_box * 105));
+  const bool flat = t.flat;
   if (flat) {
-    // rows of input one (tile, channel block) needs: one box when it has at most 256 rows (the TMA
-    // limit), else one box per filter row
-    const int all_rows = (BM + (R - 1) * (Wp + 1) + 7) / 8 * 8;
-    const int nblk = all_rows <= 256 ? 1 : R;
-    const int blk_rows = all_rows <= 256 ? all_rows : (BM + R - 1 + 7) / 8 * 8;
-    // the flat plan needs one such buffer plus two filter tiles next to the fixed part; wide
-    // filters on wide images (R >= 9, or R = 7 with 256-column tiles) do not fit and take the pixel boxes
-    const long long flat_tiles_m = (flat_rows + BM - 1) / BM;
-    const int b_rows_flat = pl_flat.pair ? pl_flat.bn / 2 : pl_flat.bn;
-    const long long need = (long long)TileCfg<64, 64>::FIXED_BYTES + 2LL * b_rows_flat * span + (long long)nblk * blk_rows * span;
-    if (need > SMEM_LIMIT) {
-      flat = false;
-    } else {
-      p.is_conv = 2;
-      p.flat_wp = Wp;
-      p.flat_hpwp = Hp * Wp;
-      division_magic(Wp, &p.magic_wp, &p.shift_wp);
-      division_magic(Hp * Wp, &p.magic_hpwp, &p.shift_hpwp);
-      p.tiles_m = (int)flat_tiles_m;
-      p.flat_nblk = nblk;
-      p.flat_blk_rows = blk_rows;
-    }
+    p.flat_wp = Wp;
+    p.flat_hpwp = Hp * Wp;
+    division_magic(Wp, &p.magic_wp, &p.shift_wp);
+    division_magic(Hp * Wp, &p.magic_hpwp, &p.shift_hpwp);
+    p.flat_nblk = t.flat_nblk;
+    p.flat_blk_rows = t.flat_blk_rows;
   }
-  const TilePlan plan = flat ? pl_flat : pl_box;
+  const int bw = t.bw, bh = t.bh, bb = t.bb;
+  const TilePlan plan = t.plan;
   const int bn = plan.bn, splits = plan.splits;
   p.pair = plan.pair;
-  if (plan.pair) p.tiles_m = (p.tiles_m + 1) / 2;   // pairs of tile rows
   CUtensorMap map_a, map_b;
   const bool maps_ok =
       (flat ? make_operand_map(&map_a, X8, flat_rows, CIN, p.flat_blk_rows, span)
@@ -1835,15 +1874,27 @@ apnn_status tc5_conv(cudaStream_t s, int wbits, int xbits, const uint32_t* Wt, c
   uint8_t* w8 = x8 + align_up((size_t)pixels * CIN, 256);
   int* err = reinterpret_cast<int*>(w8 + align_up((size_t)COUT * R * R * CIN, 256));
   const bool w_signed = epi && epi->signed_operand == APNN_SIGN_W;
-  // Operands of at most two bits as e2m1 nibbles where the flat 4-bit convolution takes the shape: half the bytes to
-  // write and read, twice the tensor rate.  (Filter rows are counted in 128-channel rows: planes and nibbles are linear.)
-  // Its tiles are 256 channels wide, so it needs more than 64 (32 x 28x28, 128 -> 64 channels: 13.4 us against 12.6 on
-  // int8; 128 -> 96 and 128 -> 128: 10.1 / 13.5 against 10.4 / 13.9), and outside the two-bit thresholds its general
-  // epilogue needs some K to hide behind (int32, 32 x 28x28, 128 -> 128: 17.2 against 12.9; 256 -> 160: 18.8 against 20.5).
+  // Operands of at most two bits as e2m1 nibbles where the flat 4-bit convolution is the faster path: half the bytes to
+  // write and read, twice the tensor rate, but tiles 256 channels wide and, as every tap of a tile reads one 256-row box of
+  // pixels, fewer pixels per tile the wider the map is (w1a2 thresholds, int8 / 4-bit, us: 4 x 90x90, 512 -> 512 channels
+  // 54 / 44, 4 x 102x102 64 / 88, 4 x 112x112 75 / 186; 47 x 6x60, 128 -> 128 9.5 / 12.5; 1x1, 37 x 45x45, 384 -> 288 36 /
+  // 56).  Both paths' times are estimated.  (Filter rows are counted in 128-channel rows: planes and nibbles are linear.)
+  // At most 64 channels stay on int8 (32 x 28x28, 128 -> 64: 13.4 us against 12.6), as does what the general epilogue has
+  // no K to hide behind (int32, 32 x 28x28, 128 -> 128: 17.2 against 12.9; 256 -> 160: 18.8 against 20.5).
   const bool thr2 = epi && epi->out_mode == APNN_OUT_THRESHOLDS && epi->out_bits <= 2 && !epi->residual_in && !epi->residual_out;
   static const bool fp4_on = [] { const char* v = getenv("APNN_FP4"); return !(v && v[0] == '0'); }();
-  if (fp4_on && wbits <= 2 && xbits <= 2 && stride == 1 && CIN % 128 == 0 && COUT > 64 && (thr2 || R * R * CIN >= 2048) && (!epi || epi->pool == APNN_POOL_NONE) &&
-      tc5_conv_fp4_clocks(B, H, W, CIN, COUT, R, pad, epi ? epi->out_halo : 0) != 0) {
+  auto fp4_faster = [&] {
+    const double us4 = tc5_conv_fp4_us(B, H, W, CIN, COUT, R, pad, epi ? epi->out_halo : 0, thr2);
+    const int sms = device_sm_count();
+    ConvTiling t;
+    if (us4 < 0.0 || !plan_conv(B, H, W, H + 2 * pad, W + 2 * pad, CIN, COUT, R, 1, APNN_POOL_NONE, false, sms, &t)) return false;
+    const double elements = (double)(pixels + (long long)COUT * R * R) * CIN;
+    // (within the estimates' error the 4-bit path: of 1826 timed convolutions 46 then run 10 % or more slower than on the
+    // other path, the worst 1.5 times, against 173 and 3.6 times when every shape it accepts took it)
+    return us4 <= 1.05 * i8_path_us(t.plan, t.tiles_m, COUT, R * R * (CIN / 128), elements, sms, t.flat ? 0.031 : 0.179, 1.3);
+  };
+  if (fp4_on && wbits <= 2 && xbits <= 2 && stride == 1 && CIN % 128 == 0 && COUT > 64 && (thr2 || R * R * CIN >= 2048) &&
+      (!epi || epi->pool == APNN_POOL_NONE) && fp4_faster()) {
     apnn_status s4 = tc5_expand2_fp4(s, X, x8, pixels * (CIN / 128), xbits, false, Wt, w8, (long long)COUT * R * R * (CIN / 128),
                                      wbits, w_signed, 128);
     if (s4 != APNN_OK) return s4;

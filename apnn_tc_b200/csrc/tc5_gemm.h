@@ -42,8 +42,10 @@ apnn_status tc5_expand_fp4(cudaStream_t s, const uint32_t* planes, uint8_t* out,
 apnn_status tc5_expand2_fp4(cudaStream_t s, const uint32_t* pa, uint8_t* oa, long long rows_a, int bits_a, bool signed_a,
                             const uint32_t* pb, uint8_t* ob, long long rows_b, int bits_b, bool signed_b, int K);
 // Stride-1 convolution over e2m1 nibble rows (tc5_fp4.cu): R in {1, 3}, CIN % 128 == 0, no pooling, any output mode;
-// epi->out_i8 = 2 writes nibble rows.  The estimate is in SM clocks, 0 for shapes it does not take.
+// epi->out_i8 = 2 writes nibble rows.  tc5_conv_fp4_clocks: the tile plan's estimate in SM clocks, 0 for shapes it does not
+// take; tc5_conv_fp4_us: expand pass and convolution together, to compare with the int8 path, negative for such shapes.
 long long tc5_conv_fp4_clocks(int B, int H, int W, int CIN, int COUT, int R, int in_halo, int out_halo);
+double tc5_conv_fp4_us(int B, int H, int W, int CIN, int COUT, int R, int in_halo, int out_halo, bool thr2);
 apnn_status tc5_conv_fp4(cudaStream_t s, const uint8_t* X4, const uint8_t* W4, void* Out, int B, int H, int W, int CIN,
                          int COUT, int R, const apnn_epilogue* epi, int* status_flag);
 // The GEMM on the same kernel (any M and N, K % 128 == 0): narrow tiles and split K for problems of few tiles.

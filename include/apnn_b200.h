@@ -270,9 +270,9 @@ apnn_status apnn_conv2d_i8(void *stream, const void *W8, const void *X8, void *O
 /* The stride-1 convolution of apnn_conv2d_i8 on operands of at most two bits in e2m1 nibbles (see
  * apnn_expand_planes_fp4; filter rows W4[COUT][R*R*CIN/2], activations X4[B][H+2h][W+2h][CIN/2]) at
  * twice the int8 tensor rate, bit for bit the same results.  R is 1 or 3, CIN % 128 == 0, the sums
- * stay below 2^24 (9*R*R*CIN < 2^24), no pooling, no APNN_OUT_FLOAT, and the image is at most about
- * 100 pixels wide for R = 3 (the rows the taps of a tile reach must fit one 256-row box), else
- * APNN_ERR_UNSUPPORTED.  epi->out_i8 = 1 writes int8 rows, APNN_ROWS_FP4 nibble rows (out_bits <= 2):
+ * stay below 2^24 (9*R*R*CIN < 2^24), no pooling, no APNN_OUT_FLOAT, and for R = 3 the stored rows are at
+ * most 119 pixels wide (the rows the taps of a tile reach must fit one 256-row box), else
+ * APNN_ERR_UNSUPPORTED.  Above 100 pixels the box leaves so few pixels per tile that apnn_conv2d_i8 is faster.  epi->out_i8 = 1 writes int8 rows, APNN_ROWS_FP4 nibble rows (out_bits <= 2):
  * the operand of the next such layer.  No reference counterpart. */
 #define APNN_ROWS_FP4 2
 apnn_status apnn_conv2d_fp4(void *stream, const void *W4, const void *X4, void *Out, int B, int H, int W,

@@ -126,6 +126,30 @@ def test_status_flag_of_an_unaligned_workspace_is_not_stored_by_a_kernel():
                 assert L.apnn_last_cuda_error().startswith(b"status flag reset") == reset, (algo, offset)
 
 
+# us on int8 and on the 4-bit path where they were timed (expand pass and kernel): the choice takes the faster one
+CONV_ROUTES = [
+    # B, H, W, CIN, COUT, R, output, int8, 4-bit
+    (8, 16, 16, 1024, 1024, 3, "thr", 24.0, 17.8), (4, 90, 90, 512, 512, 3, "thr", 53.8, 43.7), (4, 112, 112, 512, 512, 3, "thr", 74.7, 186.1),
+    (4, 102, 102, 512, 512, 3, "thr", 64.1, 87.8), (2, 30, 112, 256, 256, 3, "int32", 10.7, 15.2), (4, 117, 117, 384, 384, 3, "thr", 59.1, 191.2),
+    (7, 5, 110, 640, 960, 3, "thr", 24.2, 68.1), (3, 38, 38, 896, 1024, 3, "thr", 47.1, 26.5), (47, 6, 60, 128, 128, 3, "thr", 9.5, 12.5),
+    (37, 45, 45, 384, 288, 1, "thr", 36.1, 56.3), (20, 38, 38, 1024, 384, 1, "thr", 32.1, 20.6), (2, 14, 14, 1024, 352, 3, "thr", 17.1, 11.3),
+]
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host addresses stand in for device memory: only without a device")
+@pytest.mark.parametrize("B,H,W,CIN,COUT,R,out,us8,us4", CONV_ROUTES)
+def test_convolution_path_follows_the_measurements(B, H, W, CIN, COUT, R, out, us8, us4):
+    """Without a device the call ends in its first launch, the expand pass, whose name tells the operand type."""
+    L = _cabi.lib()
+    buf = (ctypes.c_uint32 * 64)()
+    base = ctypes.addressof(buf)
+    p = base + (-base % 32)
+    e = _cabi.Epilogue(out_mode=2, out_bits=2, signed_operand=1, thresholds=p) if out == "thr" else _cabi.Epilogue()
+    size = L.apnn_conv2d_workspace_bytes(3, B, H, W, CIN, COUT, R)
+    assert L.apnn_conv2d_ex(None, 3, 1, 2, p, p, p, B, H, W, CIN, COUT, R, 1, ctypes.byref(e), p, size) == 5
+    assert L.apnn_last_cuda_error().startswith(b"expand_nibbles" if us4 < us8 else b"expand_planes")
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_cabi, "_lib", None)
     monkeypatch.setattr(_cabi, "LIB_PATH", str(tmp_path / "nope.so"))

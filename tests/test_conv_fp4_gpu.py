@@ -50,6 +50,8 @@ SHAPES = [
     # more tiles than SM pairs
     (1, 2, 2, 128, 32, 3), (2, 7, 7, 512, 512, 3), (3, 13, 13, 384, 384, 3), (1, 56, 56, 256, 256, 3), (2, 5, 100, 128, 64, 3),
     (1, 1, 1, 128, 32, 1), (2, 14, 14, 256, 160, 1), (4, 9, 11, 1152, 288, 1), (24, 28, 28, 128, 512, 3),
+    # the widest maps the 256-row box takes: tiles of 64 and of 32 pixels, several waves of them
+    (2, 9, 104, 256, 96, 3), (3, 30, 117, 128, 288, 3), (2, 3, 117, 512, 160, 3),
 ]
 
 
@@ -220,3 +222,20 @@ def test_gemm_on_narrow_tiles_and_split_k(cuda_device, M, N, K, sign):
         out = linear(torch.zeros((M, N // form), dtype=torch.uint8, device="cuda"),
                      ap.make_epilogue("thresholds", 2, thresholds=to_dev(T), out_i8=form)).cpu().numpy()
         assert np.array_equal(out, spread_bytes(lv) if form == 1 else spread_nibbles(lv))
+
+
+@pytest.mark.parametrize("H,Wd", [(6, 100), (5, 101), (4, 108), (5, 117), (3, 118)])
+@pytest.mark.parametrize("CIN,COUT", [(128, 256), (512, 96)])
+def test_wide_maps_from_planes(cuda_device, H, Wd, CIN, COUT):
+    """Around the width where packed planes go to int8 instead, and beyond what the 4-bit kernel takes."""
+    import apnn_tc_b200 as ap
+    rng = np.random.default_rng(Wd)
+    X, Wt = make_conv(rng, 2, H, Wd, CIN, COUT, 3, 1, 2)
+    v = oracle.conv_popc(Wt, X, threads=8)
+    ws = torch.empty(ap.conv_workspace_bytes(2, H, Wd, CIN, COUT, 3), dtype=torch.uint8, device="cuda")
+    got = ap.apconv(to_dev(Wt), to_dev(X), algo="tcgen05", workspace=ws)
+    assert np.array_equal(to_host(got, np.int32), v)
+    v = oracle.signed_correct(v, oracle.conv_window_sums(X, 3), 0)
+    T = oracle.fold_bn(np.ones(COUT, np.float32), np.zeros(COUT, np.float32), float(v.mean()), float(v.std()) / 4, 2)
+    got = ap.apconv(to_dev(Wt), to_dev(X), algo="tcgen05", workspace=ws, epilogue=ap.make_epilogue("thresholds", 2, signed="w", thresholds=to_dev(T)))
+    assert np.array_equal(to_host(got), oracle.requant_pack(v, 2, 2, T))
