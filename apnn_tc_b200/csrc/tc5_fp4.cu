@@ -533,13 +533,14 @@ long long tc5_conv_fp4_clocks(int B, int Hin, int Win, int CIN, int COUT, int R,
 // 120) and 992 GEMMs timed on both paths, standard deviation 9 %: launches; 0.19 ns per 1000 elements expanded; per
 // tile 0.5 us and its K blocks, whose 64-byte rows (CIN % 256 != 0) arrive at half the rate; the last tile's epilogue, 32
 // pixels of a warp at a time.  thr2: thresholds of at most two bits, no residuals.
-double tc5_conv_fp4_us(int B, int Hin, int Win, int CIN, int COUT, int R, int in_halo, int out_halo, bool thr2) {
+double tc5_conv_fp4_us(int B, int Hin, int Win, int CIN, int COUT, int R, int in_halo, int out_halo, bool thr2, long long* waves) {
   if (!fp4_takes(B, Hin, Win, CIN, R, in_halo, out_halo)) return -1.0;
   const int Hp = Hin + 2 * in_halo, Wp = Win + 2 * in_halo;
   const long long flat_rows = (long long)B * Hp * Wp;
   const int span = CIN % 256 == 0 ? 128 : 64;
   const Fp4Plan pl = plan_np(flat_rows, COUT, R, Wp, CIN / 2, span, device_sm_count());
   if (pl.np == 0) return -1.0;
+  if (waves) *waves = pl.waves;
   const double elements = (double)(flat_rows + (long long)COUT * R * R) * CIN;
   const int kblocks = (CIN / 2 / span + pl.splits - 1) / pl.splits;
   const double bytes = (double)span * (R * R * HALF + box_rows_of(R, Wp, pl.np));   // operand bytes of a K block

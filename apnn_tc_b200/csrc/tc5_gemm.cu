@@ -1619,6 +1619,23 @@ apnn_status tc5_gemm_i8(cudaStream_t s, const uint8_t* A8, const uint8_t* B8, vo
   return APNN_OK;
 }
 
+namespace {
+
+// Time of the expand pass and the int8 kernel together in us, to compare with tc5_conv_fp4_us; fitted to the same
+// timings (standard deviation 9 %).  tiles_m: tile rows (pairs of them when plan.pair); row_ns: per operand row of a K
+// block; base_us: what a convolution's launch takes more than a GEMM's.
+double i8_path_us(const TilePlan& plan, long long tiles_m, int N, int kblocks, double elements, int sms, double row_ns,
+                  double base_us) {
+  const long long units = tiles_m * ((N + plan.bn - 1) / plan.bn) * plan.splits, slots = plan.pair ? sms / 2 : sms;
+  const long long waves = (units + slots - 1) / slots;
+  const int rows = BM + (plan.pair ? plan.bn / 2 : plan.bn);
+  const double loop_ns = ((kblocks + plan.splits - 1) / plan.splits) * (217.0 + rows * row_ns), drain_ns = 2.5 * plan.bn;
+  return base_us + 0.21e-6 * elements + waves * (2.5 + 1e-3 * (loop_ns > drain_ns ? loop_ns : drain_ns)) + 0.0205 * plan.bn +
+         (plan.splits > 1 ? 3.6 : 0.0);
+}
+
+}  // namespace
+
 apnn_status tc5_gemm(cudaStream_t s, int wbits, int xbits, const uint32_t* W, const uint32_t* X, void* D, int M,
                      int N, int K, const apnn_epilogue* epi, void* workspace, int pair) {
   uint8_t* wa = reinterpret_cast<uint8_t*>(workspace);
@@ -1636,12 +1653,21 @@ apnn_status tc5_gemm(cudaStream_t s, int wbits, int xbits, const uint32_t* W, co
     return tc5_gemm_fp4_pair(s, wa, xb4, D, M, N, K, epi, err);
   }
   // problems with fewer tiles than that: the flat 4-bit kernel, whose tile width and K split follow the shape, for the
-  // two-bit thresholds it packs cheaply (128 x 4096 x 9216: 18.3 us against 22.1 on int8; 2048^3 16.3 / 15.1, 1024 x 1024 x
-  // 2048 11.2 / 12.9; int32 rows 2048^3 17.9 / 13.6)
+  // two-bit thresholds it packs cheaply, where its estimated time is not above int8's.  Tiles of one wave with a long K gain;
+  // a second wave of long tiles (which the estimate takes for shorter than it is) and K = 128 mod 256 (64-byte rows) lose (int8 / 4-bit, us: 1792 x 2048 x 4096 21.0 / 17.0, 1024 x 1024 x 2048
+  // 12.7 / 11.1, 2048^3 15.2 / 16.1, 2048 x 2048 x 4096 21.0 / 23.4, 7040 x 64 x 256 5.5 / 8.8; int32 rows 2048^3 13.6 / 17.9).
+  // Of 992 timed shapes 14 then run 10 % or more slower than on the other path, 171 when all of them took it.
   const bool thr2 = epi && epi->out_mode == APNN_OUT_THRESHOLDS && epi->out_bits <= 2 && !epi->residual_in && !epi->residual_out &&
                     epi->n_peer_out == 0;
-  if (fp4_on && wbits <= 2 && xbits <= 2 && !pair && thr2 && !takes_pair_kernel(M, N, K, epi) &&
-      tc5_gemm_fp4_flat_clocks(M, N, K) != 0) {
+  auto flat_faster = [&] {
+    long long waves = 0;
+    const double us4 = tc5_conv_fp4_us(1, 1, M, K, N, 1, 0, 0, true, &waves);   // one tap: rows of W as pixels, rows of X as channels
+    const int sms = device_sm_count(), tiles_m = (M + BM - 1) / BM;
+    const TilePlan plan = pick_plan(tiles_m, N, K / BK, sms, pick_bn(tiles_m, N, sms), true);
+    return us4 >= 0.0 && (waves == 1 || K <= 1024) && us4 <= i8_path_us(plan, plan.pair ? (tiles_m + 1) / 2 : tiles_m, N, K / BK, (double)(M + (long long)N) * K, sms,
+                                           0.431, 0.0);
+  };
+  if (fp4_on && wbits <= 2 && xbits <= 2 && !pair && thr2 && !takes_pair_kernel(M, N, K, epi) && flat_faster()) {
     uint8_t* xb4 = wa + align_up((size_t)M * (K / 2), 256);
     apnn_status s4 = tc5_expand2_fp4(s, W, wa, M, wbits, sign == APNN_SIGN_W, X, xb4, N, xbits, sign == APNN_SIGN_X, K);
     if (s4 != APNN_OK) return s4;
@@ -1761,19 +1787,6 @@ bool plan_conv(int B, int H, int W, int Hp, int Wp, int CIN, int COUT, int R, in
   t->tiles_m = t->flat ? flat_tiles_m : tiles_m_box;
   if (t->plan.pair) t->tiles_m = (t->tiles_m + 1) / 2;
   return true;
-}
-
-// Time of the expand pass and the int8 kernel together in us, to compare with tc5_conv_fp4_us; fitted to the same
-// timings (standard deviation 9 %).  tiles_m: tile rows (pairs of them when plan.pair); row_ns: per operand row of a K
-// block; base_us: what a convolution's launch takes more than a GEMM's.
-double i8_path_us(const TilePlan& plan, long long tiles_m, int N, int kblocks, double elements, int sms, double row_ns,
-                  double base_us) {
-  const long long units = tiles_m * ((N + plan.bn - 1) / plan.bn) * plan.splits, slots = plan.pair ? sms / 2 : sms;
-  const long long waves = (units + slots - 1) / slots;
-  const int rows = BM + (plan.pair ? plan.bn / 2 : plan.bn);
-  const double loop_ns = ((kblocks + plan.splits - 1) / plan.splits) * (217.0 + rows * row_ns), drain_ns = 2.5 * plan.bn;
-  return base_us + 0.21e-6 * elements + waves * (2.5 + 1e-3 * (loop_ns > drain_ns ? loop_ns : drain_ns)) + 0.0205 * plan.bn +
-         (plan.splits > 1 ? 3.6 : 0.0);
 }
 
 }  // namespace

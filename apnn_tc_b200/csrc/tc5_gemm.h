@@ -45,7 +45,8 @@ apnn_status tc5_expand2_fp4(cudaStream_t s, const uint32_t* pa, uint8_t* oa, lon
 // epi->out_i8 = 2 writes nibble rows.  tc5_conv_fp4_clocks: the tile plan's estimate in SM clocks, 0 for shapes it does not
 // take; tc5_conv_fp4_us: expand pass and convolution together, to compare with the int8 path, negative for such shapes.
 long long tc5_conv_fp4_clocks(int B, int H, int W, int CIN, int COUT, int R, int in_halo, int out_halo);
-double tc5_conv_fp4_us(int B, int H, int W, int CIN, int COUT, int R, int in_halo, int out_halo, bool thr2);
+double tc5_conv_fp4_us(int B, int H, int W, int CIN, int COUT, int R, int in_halo, int out_halo, bool thr2,
+                       long long* waves = nullptr);
 apnn_status tc5_conv_fp4(cudaStream_t s, const uint8_t* X4, const uint8_t* W4, void* Out, int B, int H, int W, int CIN,
                          int COUT, int R, const apnn_epilogue* epi, int* status_flag);
 // The GEMM on the same kernel (any M and N, K % 128 == 0): narrow tiles and split K for problems of few tiles.

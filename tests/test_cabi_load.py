@@ -150,6 +150,26 @@ def test_convolution_path_follows_the_measurements(B, H, W, CIN, COUT, R, out, u
     assert L.apnn_last_cuda_error().startswith(b"expand_nibbles" if us4 < us8 else b"expand_planes")
 
 
+GEMM_ROUTES = [   # M, N, K, us on int8, us on the flat 4-bit kernel: two-bit thresholds, expand pass and kernel
+    (1792, 2048, 4096, 21.0, 17.0), (1024, 1024, 4096, 18.7, 14.4), (512, 512, 9216, 17.5, 13.9), (8000, 256, 9216, 38.0, 26.9),
+    (2048, 2048, 4096, 21.0, 23.4), (2048, 2304, 2048, 15.0, 16.8), (2048, 2048, 2048, 15.2, 16.1), (7040, 64, 256, 5.5, 8.8),
+    (984, 2304, 128, 6.9, 8.4), (2240, 1920, 640, 10.7, 13.7),
+]
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host addresses stand in for device memory: only without a device")
+@pytest.mark.parametrize("M,N,K,us8,us4", GEMM_ROUTES)
+def test_threshold_gemm_path_follows_the_measurements(M, N, K, us8, us4):
+    L = _cabi.lib()
+    buf = (ctypes.c_uint32 * 64)()
+    base = ctypes.addressof(buf)
+    p = base + (-base % 32)
+    e = _cabi.Epilogue(out_mode=2, out_bits=2, signed_operand=1, thresholds=p)
+    size = L.apnn_gemm_workspace_bytes(3, 1, 2, M, N, K)
+    assert L.apnn_gemm_ex(None, 3, 1, 2, p, p, p, M, N, K, ctypes.byref(e), p, size) == 5
+    assert L.apnn_last_cuda_error().startswith(b"expand_nibbles" if us4 < us8 else b"expand_planes")
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_cabi, "_lib", None)
     monkeypatch.setattr(_cabi, "LIB_PATH", str(tmp_path / "nope.so"))

@@ -176,7 +176,7 @@ def test_int8_layer_writes_nibble_rows(cuda_device, CIN, COUT, R, stride, mode, 
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 32, 128), (128, 4096, 2304), (64, 512, 9216), (200, 96, 1280), (33, 1000, 4096), (8, 512, 25088),
-                                   (2300, 352, 640)])
+                                   (2300, 352, 640), (1175, 288, 896), (1024, 1024, 1280), (2240, 1920, 640)])
 @pytest.mark.parametrize("sign", ["none", "w", "x"])
 def test_gemm_on_narrow_tiles_and_split_k(cuda_device, M, N, K, sign):
     """apnn_linear_fp4 (split K, ragged edges, every output form) and apmm on tcgen05 below the CTA-pair kernel's size."""
