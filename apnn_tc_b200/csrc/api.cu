@@ -259,7 +259,10 @@ apnn_status apnn_gemm_ex(void* stream, int algo, int wbits, int xbits, const voi
     // operand the expand pass would write and read for few uses (int32, us: 2048 x 2048 x 256 8.3 against 12.2 on the
     // warp-level kernel, packed output 11.5 / 27.2; 8192 x 512 x 512 9.3 / 12.1; but 64 x 4096 x 4096 14.3 / 9.5)
     // (The second kind also has a warp-level kernel, which takes a workspace of any alignment.)
-    const bool mid = aligned32(workspace) && M >= 512 && N >= 512 && 2.0 * M * N * K >= 2e9;
+    // int32 rows that are not whole 16-byte pieces the tcgen05 kernels store element by element: the warp-level kernel then
+    // (1612 x 5887 x 256 64.5 against 27.5, 7160 x 1066 x 512 50.9 / 21.8, w1a4 2030 x 2970 x 256 47.3 / 25.9).
+    const bool int32_out = !epi || epi->out_mode == APNN_OUT_INT32;
+    const bool mid = aligned32(workspace) && M >= 512 && N >= 512 && 2.0 * M * N * K >= 2e9 && !(int32_out && N % 4 != 0);
     algo = (ws_ok && (tc5_worthwhile(M, N, K) || mid || !warp_ok)) ? APNN_ALGO_TCGEN05 : APNN_ALGO_IMMA;
   }
   if (!warp_ok && algo != APNN_ALGO_TCGEN05 && algo != APNN_ALGO_TCGEN05_PAIR)

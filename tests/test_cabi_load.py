@@ -170,6 +170,20 @@ def test_threshold_gemm_path_follows_the_measurements(M, N, K, us8, us4):
     assert L.apnn_last_cuda_error().startswith(b"expand_nibbles" if us4 < us8 else b"expand_planes")
 
 
+@pytest.mark.skipif(torch.cuda.is_available(), reason="host addresses stand in for device memory: only without a device")
+@pytest.mark.parametrize("wbits,xbits,M,N,K,warp", [(1, 2, 1612, 5887, 256, True), (1, 1, 5670, 1526, 256, True), (1, 4, 2030, 2970, 256, True),
+                                                    (2, 2, 2485, 7156, 512, False), (1, 3, 1612, 5888, 256, False), (1, 2, 4096, 4097, 1024, False)])
+def test_automatic_choice_for_ragged_int32_rows(wbits, xbits, M, N, K, warp):
+    """Rows of N % 4 != 0 integers stay on the warp-level kernel below the device-filling size (4096 x 4097 x 1024 is above)."""
+    L = _cabi.lib()
+    buf = (ctypes.c_uint32 * 64)()
+    base = ctypes.addressof(buf)
+    p = base + (-base % 32)
+    size = L.apnn_gemm_workspace_bytes(3, wbits, xbits, M, N, K)
+    assert L.apnn_gemm_ex(None, 0, wbits, xbits, p, p, p, M, N, K, None, p, size) == 5
+    assert L.apnn_last_cuda_error().startswith(b"apnn_gemm launch" if warp else b"expand_")
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_cabi, "_lib", None)
     monkeypatch.setattr(_cabi, "LIB_PATH", str(tmp_path / "nope.so"))
