@@ -84,6 +84,41 @@ cudaError_t ensure_max_smem(const void* kernel, int bytes) {
   return e;
 }
 
+int cluster_capacity(const void* kernel, int threads, int smem, int ctas) {
+  struct Entry {
+    const void* kernel;
+    int ctas, dev, n;
+  };
+  static std::mutex mu;
+  static std::vector<Entry> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  for (const Entry& k : known)
+    if (k.kernel == kernel && k.ctas == ctas && k.dev == dev) return k.n;
+  int n = 0;
+  if (ensure_max_smem(kernel, smem) == cudaSuccess) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)(ctas * device_sm_count()), 1, 1);
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      n = 0;
+    }
+  }
+  known.push_back({kernel, ctas, dev, n});
+  return n;
+}
+
 void* tensor_map_encoder() {
   static std::once_flag once;
   static void* fn = nullptr;
@@ -387,7 +422,7 @@ apnn_status apnn_gemm_planes(void* stream, int wbits, int xbits, const void* W, 
   if (K % 128 != 0 || !aligned16(W) || !aligned16(X) || !aligned16(D)) return APNN_ERR_ALIGNMENT;
   apnn_status st = check_epilogue(epi, N, false, wbits, xbits);
   if (st != APNN_OK) return st;
-  if ((epi && epi->n_peer_out != 0) || tc5_gemm_planes_clocks(wbits, xbits, M, N, K) == 0) return APNN_ERR_UNSUPPORTED;
+  if ((epi && epi->n_peer_out != 0) || !tc5_gemm_planes_takes(wbits, xbits, K)) return APNN_ERR_UNSUPPORTED;
   return tc5_gemm_planes(reinterpret_cast<cudaStream_t>(stream), wbits, xbits, (const uint32_t*)W, (const uint32_t*)X, D, M, N,
                          K, epi, status_flag);
 }

@@ -12,6 +12,9 @@ apnn_status check_epilogue(const apnn_epilogue* e, int channels, bool is_conv, i
                            bool i8_rows_ok = false, bool fp4_rows_ok = false);
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per (kernel, device); safe to call from several threads.
 cudaError_t ensure_max_smem(const void* kernel, int bytes);
+// How many clusters of `ctas` CTAs of a kernel with `smem` bytes of dynamic shared memory the device holds at once (0 on
+// error); asked of the driver once per (kernel, ctas, device).
+int cluster_capacity(const void* kernel, int threads, int smem, int ctas);
 // Address of the driver's cuTensorMapEncodeTiled (null if unavailable); looked up once, thread-safe.
 void* tensor_map_encoder();
 // Launch attribute for programmatic dependent launch: writes it to attrs[0] and returns 1, or

@@ -53,8 +53,8 @@ apnn_status tc5_conv_fp4(cudaStream_t s, const uint8_t* X4, const uint8_t* W4, v
 long long tc5_gemm_fp4_flat_clocks(int M, int N, int K);
 apnn_status tc5_gemm_fp4_flat(cudaStream_t s, const uint8_t* A4, const uint8_t* B4, void* D, int M, int N, int K,
                               const apnn_epilogue* epi, int* status_flag);
-// GEMM of 1- and 2-bit operands from their packed planes in one launch (tc5_planes.cu); estimate in SM clocks, 0: not taken.
-long long tc5_gemm_planes_clocks(int wbits, int xbits, int M, int N, int K);
+// GEMM of 1- and 2-bit operands from their packed planes in one launch (tc5_planes.cu).
+bool tc5_gemm_planes_takes(int wbits, int xbits, int K);
 bool tc5_gemm_planes_preferred(int wbits, int xbits, int M, int N, int K, bool packed_out);
 apnn_status tc5_gemm_planes(cudaStream_t s, int wbits, int xbits, const uint32_t* W, const uint32_t* X, void* D, int M, int N,
                             int K, const apnn_epilogue* epi, int* status_flag);

@@ -15,7 +15,7 @@
 // took 1400 clk).  One more thread issues the MMAs.  The operands need no cluster, so all those barriers are local.
 //
 // What bounds it: launch, first box, exchange and epilogue, 4 to 5 us together; then the spreading, about 0.5 us per K block
-// (128 x 4096 x 9216, thresholds: 13.2 us, 33.1 on the warp-level kernel; 64 x 128 x 128: 3.7 against 7.5).
+// (128 x 4096 x 9216, thresholds: 13.4 us, 33.5 on the warp-level kernel; 64 x 128 x 128: 3.7 against 7.5).
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -340,30 +340,39 @@ tc5_planes_kernel(const __grid_constant__ CUtensorMap map_px, const __grid_const
 
 struct PlanesPlan {
   int np, splits;
-  long long clk;
+  double us;   // estimated time, launch included
 };
-// Tile width and K split.  Per K block a CTA writes and reads (128 + np) rows of 128 bytes in shared memory; per tile it pays
-// the first loads, the pipeline's tail and the epilogue; clusters must all be resident (70 of 2, 33 of 4, 15 of 8 CTAs at most).
 // Shared memory besides the operand stages.
 int fixed_bytes(int pxb, int chb, int np) { return 1024 + BAR_BYTES + ROWS_BYTES + RAW_STAGES * (chb * HALF + pxb * np) * 128; }
 int stages_of(int pxb, int chb, int np) {
   const int n = (SMEM_LIMIT - fixed_bytes(pxb, chb, np)) / (CH_BYTES + np * 128);
   return n < MAX_STAGES ? n : MAX_STAGES;
 }
+// Tile width and K split of the shortest estimated time; a split needs all its clusters resident.  The estimate is fitted to
+// 2531 timed one-wave problems of w1a1, w1a2, w2a1 and w2a2 (standard deviation 9 %, split ones 4 %): per K block of 256 the
+// planes to fetch and spread and the pixel columns to multiply; 32-pixel chunks of the epilogue, a warp's share of them
+// one after the other; of a split the partial sums a warp sends away (1.2 us per chunk) and, per chunk kept, those it adds
+// (0.46 us for each other CTA).  When sending cost a constant instead, wide tiles split eight ways were chosen: w1a1, 512 x
+// 512 x 4096 took 12.7 us on 192 columns and 8 CTAs, 8.3 on 64 and 4.
 PlanesPlan plan_planes(int pxb, int chb, int M, int N, int K, int sms) {
-  PlanesPlan best = {0, 1, 0};
-  const long long kblocks = (K + KB - 1) / KB;
+  PlanesPlan best = {0, 1, 0.0};
+  const int kblocks = (K + KB - 1) / KB;
   const long long tiles_n = (N + HALF - 1) / HALF;
   for (int splits = 1; splits <= 8; splits *= 2) {
     if (splits > 1 && kblocks < 2 * splits) break;
+    const int resident = splits == 1 ? 0 : cluster_capacity(reinterpret_cast<const void*>(tc5_planes_kernel<2, 2, 1, true>), THREADS, SMEM_LIMIT, splits);
     for (int np = 32; np <= MAX_NP; np += 32) {
       if (stages_of(pxb, chb, np) < 2) continue;
       const long long tiles = (((long long)M + np - 1) / np) * tiles_n;
-      if (splits > 1 && (tiles * splits > sms || (splits > 1 && tiles > (splits == 2 ? 70 : splits == 4 ? 33 : 15)))) continue;
+      if (splits > 1 && tiles > resident) continue;
       const long long waves = (tiles * splits + sms - 1) / sms;
-      const long long per = (HALF + np) * 9LL / 4 + 60;
-      const long long clk = waves * ((kblocks + splits - 1) / splits * per + 2500 + 12LL * np / splits) + (splits > 1 ? 2000 : 0) + 2500;
-      if (best.np == 0 || clk < best.clk) best = {np, splits, clk};
+      const int chunks = np / 32, per_warp = WORKERS / 4;
+      const int kept = ((chunks + splits - 1) / splits + per_warp - 1) / per_warp;
+      const int sent = (chunks * (splits - 1) + splits * per_warp - 1) / (splits * per_warp);
+      const double block = 0.22 + 0.0009 * np + 0.113 * (pxb * np + chb * HALF) / HALF;
+      const double tile = ((kblocks + splits - 1) / splits) * block + kept * (1.13 + 0.46 * (splits - 1)) + 1.18 * sent;
+      const double us = waves * (2.5 + tile);   // a further wave pays its set-up and first loads again
+      if (best.np == 0 || us < best.us) best = {np, splits, us};
     }
   }
   return best;
@@ -430,30 +439,29 @@ cudaError_t launch_bits(cudaStream_t s, const CUtensorMap& mp, const CUtensorMap
 
 }  // namespace
 
-long long tc5_gemm_planes_clocks(int wbits, int xbits, int M, int N, int K) {
-  if (wbits < 1 || wbits > 2 || xbits < 1 || xbits > 2 || K % 128 != 0 || (long long)K * 9 >= (1ll << 24)) return 0;
-  return plan_planes(wbits, xbits, M, N, K, device_sm_count()).clk;
+bool tc5_gemm_planes_takes(int wbits, int xbits, int K) {
+  return wbits >= 1 && wbits <= 2 && xbits >= 1 && xbits <= 2 && K % 128 == 0 && (long long)K * 9 < (1ll << 24);
 }
 
-// Whether the kernel is the fastest way to run the problem, measured on w1a2 (us: this kernel / warp-level / expand pass and
-// tcgen05).  It needs one wave of tiles with at most a dozen K blocks each (thresholds, 128 x 4096 x 9216: 13.2 / 33.1 /
-// 22.1; 2048 x 1024 x 1024: 6.7 / 30.0 / 9.6; 8192 x 64 x 2048: 7.9 / 12.2 / 11.6; two waves, 2048 x 2048 x 512: 10.5 / 27.3
-// / 9.6).  Packed outputs then always gain (64 x 1024 x 1024: 5.0 / 8.7 / 6.8): the warp-level epilogue takes about 4 us.
-// For int32 the warp-level kernel, about 3.2 us + 1.5 us per 1024 k and wave of its 64 x 32 tiles, keeps the smallest
+// Whether the kernel is the fastest way to run the problem (us: this kernel / warp-level / expand pass and tcgen05).  It
+// needs one wave of tiles with at most 24 K blocks each (thresholds, 128 x 4096 x 9216: 13.4 / 33.5 / 21.9; 2048 x 1024 x
+// 1024: 6.7 / 30.0 / 9.6; 8192 x 64 x 2048: 8.6 / 12.2 / 11.8; two waves, 2048 x 2048 x 512: 10.5 / 27.3 / 9.6; 25 to 40 K
+// blocks 0.82 to 1.3 times as fast as the best other way).  Packed outputs then always gain (64 x 1024 x 1024: 5.0 / 8.7 /
+// 6.8): the warp-level epilogue takes about 4 us.  For int32 the warp-level kernel, about 2.9 us + 0.4 us and 0.4 us per
+// 1024 k and plane for each wave of its 64 x 32 tiles (645 problems of w1a1, w1a2, w2a1 and w2a2), keeps the smallest
 // (64 x 1024 x 1024: 5.2 / 4.5; 1024 x 1024 x 512: 4.9 / 5.6).
 bool tc5_gemm_planes_preferred(int wbits, int xbits, int M, int N, int K, bool packed_out) {
   static const bool fp4_on = [] { const char* v = getenv("APNN_FP4"); return !(v && v[0] == '0'); }();
-  if (!fp4_on || tc5_gemm_planes_clocks(wbits, xbits, M, N, K) == 0) return false;
+  if (!fp4_on || !tc5_gemm_planes_takes(wbits, xbits, K)) return false;
   const int sms = device_sm_count();
   const PlanesPlan pl = plan_planes(wbits, xbits, M, N, K, sms);
   const long long tiles = (((long long)M + pl.np - 1) / pl.np) * ((N + HALF - 1) / HALF);
   const int blocks = ((K + KB - 1) / KB + pl.splits - 1) / pl.splits;
-  if (tiles * pl.splits > sms || blocks > 12) return false;
+  if (tiles * pl.splits > sms || blocks > 24) return false;
   if (packed_out) return true;
-  const double warp_tiles = (double)((M + 63) / 64) * ((N + 31) / 32) / (1.05 * sms);
-  const double warp_us = 3.2 + 1.5 * K / 1024.0 * (warp_tiles > 1.0 ? warp_tiles : 1.0);
-  const double here_us = 3.4 + 0.75 * blocks + (pl.splits > 1 ? 1.5 : 0.0);
-  return here_us < warp_us;
+  const double warp_tiles = (double)((M + 63) / 64) * ((N + 31) / 32) / sms;
+  const double warp_us = 2.9 + (warp_tiles > 1.0 ? warp_tiles : 1.0) * (0.4 + K / 1024.0 * (0.39 * (wbits + xbits) + 0.37));
+  return pl.us < warp_us;
 }
 
 apnn_status tc5_gemm_planes(cudaStream_t s, int wbits, int xbits, const uint32_t* W, const uint32_t* X, void* D, int M, int N,

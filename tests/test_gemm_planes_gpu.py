@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 # one piece of K, half a K block at the end, partial tiles in both directions, widths of the pixel tile, split K over
 # clusters of 2, 4 and 8, several waves
 SHAPES = [(1, 1, 128), (31, 33, 384), (64, 128, 128), (100, 96, 640), (129, 257, 1024), (224, 512, 2048), (64, 1024, 8192),
-          (128, 4096, 9216), (64, 128, 16384), (700, 416, 1152), (2048, 1056, 256)]
+          (128, 4096, 9216), (64, 128, 16384), (700, 416, 1152), (2048, 1056, 256), (512, 512, 4096), (300, 2304, 6144), (2100, 1700, 1024)]
 
 
 def run(W, X, out, epi, wb, xb, M, N, K):
