@@ -295,9 +295,12 @@ apnn_status apnn_gemm_ex(void* stream, int algo, int wbits, int xbits, const voi
     // warp-level kernel, packed output 11.5 / 27.2; 8192 x 512 x 512 9.3 / 12.1; but 64 x 4096 x 4096 14.3 / 9.5)
     // (The second kind also has a warp-level kernel, which takes a workspace of any alignment.)
     // int32 rows that are not whole 16-byte pieces the tcgen05 kernels store element by element: the warp-level kernel then
-    // (1612 x 5887 x 256 64.5 against 27.5, 7160 x 1066 x 512 50.9 / 21.8, w1a4 2030 x 2970 x 256 47.3 / 25.9).
+    // (1612 x 5887 x 256 64.5 against 27.5, 7160 x 1066 x 512 50.9 / 21.8, w1a4 2030 x 2970 x 256 47.3 / 25.9).  Other int32
+    // rows where the estimates say so (w1a1 512 x 512 x 4096 11.7 / 8.5; w1a3 1024 x 512 x 2048 11.4 / 9.3, 2048 x 2048 x 256
+    // 8.3 / 12.5).
     const bool int32_out = !epi || epi->out_mode == APNN_OUT_INT32;
-    const bool mid = aligned32(workspace) && M >= 512 && N >= 512 && 2.0 * M * N * K >= 2e9 && !(int32_out && N % 4 != 0);
+    const bool mid = aligned32(workspace) && M >= 512 && N >= 512 && 2.0 * M * N * K >= 2e9 &&
+                     (!int32_out || (N % 4 == 0 && tc5_gemm_i8_us(M, N, K) < core_gemm_us(wbits, xbits, M, N, K, device_sm_count())));
     algo = (ws_ok && (tc5_worthwhile(M, N, K) || mid || !warp_ok)) ? APNN_ALGO_TCGEN05 : APNN_ALGO_IMMA;
   }
   if (!warp_ok && algo != APNN_ALGO_TCGEN05 && algo != APNN_ALGO_TCGEN05_PAIR)

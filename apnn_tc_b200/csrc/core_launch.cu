@@ -23,6 +23,11 @@ int core_pick_tile(const CoreParams& p, int sm_count) {
   return big_tiles * 2 >= sm_count ? TILE_BIG : TILE_SMALL;
 }
 
+double core_gemm_us(int wbits, int xbits, int M, int N, int K, int sm_count) {
+  const double tiles = (double)((M + 63) / 64) * ((N + 31) / 32) / sm_count;
+  return 2.9 + (tiles > 1.0 ? tiles : 1.0) * (0.4 + K / 1024.0 * (0.39 * (wbits + xbits) + 0.37));
+}
+
 cudaError_t launch_core(int kind, int abits, int bbits, const CoreParams& p, cudaStream_t s, int tile_class) {
 #define APNN_CASE(AB, BB) if (abits == AB && bbits == BB) return launch_pair<AB, BB>(kind, p, s, tile_class);
   APNN_PAIRS(APNN_CASE)

@@ -1636,6 +1636,12 @@ double i8_path_us(const TilePlan& plan, long long tiles_m, int N, int kblocks, d
 
 }  // namespace
 
+double tc5_gemm_i8_us(int M, int N, int K) {
+  const int sms = device_sm_count(), tiles_m = (M + BM - 1) / BM;
+  const TilePlan plan = pick_plan(tiles_m, N, K / BK, sms, pick_bn(tiles_m, N, sms), true);
+  return i8_path_us(plan, plan.pair ? (tiles_m + 1) / 2 : tiles_m, N, K / BK, (double)(M + (long long)N) * K, sms, 0.431, 0.0);
+}
+
 apnn_status tc5_gemm(cudaStream_t s, int wbits, int xbits, const uint32_t* W, const uint32_t* X, void* D, int M,
                      int N, int K, const apnn_epilogue* epi, void* workspace, int pair) {
   uint8_t* wa = reinterpret_cast<uint8_t*>(workspace);
@@ -1662,10 +1668,7 @@ apnn_status tc5_gemm(cudaStream_t s, int wbits, int xbits, const uint32_t* W, co
   auto flat_faster = [&] {
     long long waves = 0;
     const double us4 = tc5_conv_fp4_us(1, 1, M, K, N, 1, 0, 0, true, &waves);   // one tap: rows of W as pixels, rows of X as channels
-    const int sms = device_sm_count(), tiles_m = (M + BM - 1) / BM;
-    const TilePlan plan = pick_plan(tiles_m, N, K / BK, sms, pick_bn(tiles_m, N, sms), true);
-    return us4 >= 0.0 && (waves == 1 || K <= 1024) && us4 <= i8_path_us(plan, plan.pair ? (tiles_m + 1) / 2 : tiles_m, N, K / BK, (double)(M + (long long)N) * K, sms,
-                                           0.431, 0.0);
+    return us4 >= 0.0 && (waves == 1 || K <= 1024) && us4 <= tc5_gemm_i8_us(M, N, K);
   };
   if (fp4_on && wbits <= 2 && xbits <= 2 && !pair && thr2 && !takes_pair_kernel(M, N, K, epi) && flat_faster()) {
     uint8_t* xb4 = wa + align_up((size_t)M * (K / 2), 256);

@@ -69,5 +69,7 @@ apnn_status tc5_conv_i8_pair(cudaStream_t s, const uint8_t* X8, const uint8_t* W
 int* tc5_flag_slot(void* workspace, int M, int N, int K);
 int* tc5_conv_flag_slot(void* workspace, int B, int H, int W, int CIN, int COUT, int R);
 // Flag raised by a bounded wait (0 = ran to completion); synchronises the stream.
+// Estimated time of tc5_gemm's expand pass and int8 kernel, in us.
+double tc5_gemm_i8_us(int M, int N, int K);
 int tc5_read_error_flag(cudaStream_t s, const void* workspace, int M, int N, int K);
 }  // namespace apnn

@@ -21,6 +21,7 @@
 #include <mutex>
 
 #include "api_internal.h"
+#include "core_launch.h"
 #include "fp4_epilogue.cuh"
 #include "tc5_common.cuh"
 #include "tc5_gemm.h"
@@ -447,9 +448,7 @@ bool tc5_gemm_planes_takes(int wbits, int xbits, int K) {
 // needs one wave of tiles with at most 24 K blocks each (thresholds, 128 x 4096 x 9216: 13.4 / 33.5 / 21.9; 2048 x 1024 x
 // 1024: 6.7 / 30.0 / 9.6; 8192 x 64 x 2048: 8.6 / 12.2 / 11.8; two waves, 2048 x 2048 x 512: 10.5 / 27.3 / 9.6; 25 to 40 K
 // blocks 0.82 to 1.3 times as fast as the best other way).  Packed outputs then always gain (64 x 1024 x 1024: 5.0 / 8.7 /
-// 6.8): the warp-level epilogue takes about 4 us.  For int32 the warp-level kernel, about 2.9 us + 0.4 us and 0.4 us per
-// 1024 k and plane for each wave of its 64 x 32 tiles (645 problems of w1a1, w1a2, w2a1 and w2a2), keeps the smallest
-// (64 x 1024 x 1024: 5.2 / 4.5; 1024 x 1024 x 512: 4.9 / 5.6).
+// 6.8): the warp-level epilogue takes about 4 us.  For int32 the warp-level kernel keeps the smallest (64 x 1024 x 1024: 5.2 / 4.5; 1024 x 1024 x 512: 4.9 / 5.6).
 bool tc5_gemm_planes_preferred(int wbits, int xbits, int M, int N, int K, bool packed_out) {
   static const bool fp4_on = [] { const char* v = getenv("APNN_FP4"); return !(v && v[0] == '0'); }();
   if (!fp4_on || !tc5_gemm_planes_takes(wbits, xbits, K)) return false;
@@ -459,9 +458,7 @@ bool tc5_gemm_planes_preferred(int wbits, int xbits, int M, int N, int K, bool p
   const int blocks = ((K + KB - 1) / KB + pl.splits - 1) / pl.splits;
   if (tiles * pl.splits > sms || blocks > 24) return false;
   if (packed_out) return true;
-  const double warp_tiles = (double)((M + 63) / 64) * ((N + 31) / 32) / sms;
-  const double warp_us = 2.9 + (warp_tiles > 1.0 ? warp_tiles : 1.0) * (0.4 + K / 1024.0 * (0.39 * (wbits + xbits) + 0.37));
-  return pl.us < warp_us;
+  return pl.us < core_gemm_us(wbits, xbits, M, N, K, sms);
 }
 
 apnn_status tc5_gemm_planes(cudaStream_t s, int wbits, int xbits, const uint32_t* W, const uint32_t* X, void* D, int M, int N,

@@ -172,9 +172,11 @@ def test_threshold_gemm_path_follows_the_measurements(M, N, K, us8, us4):
 
 @pytest.mark.skipif(torch.cuda.is_available(), reason="host addresses stand in for device memory: only without a device")
 @pytest.mark.parametrize("wbits,xbits,M,N,K,warp", [(1, 2, 1612, 5887, 256, True), (1, 1, 5670, 1526, 256, True), (1, 4, 2030, 2970, 256, True),
-                                                    (2, 2, 2485, 7156, 512, False), (1, 3, 1612, 5888, 256, False), (1, 2, 4096, 4097, 1024, False)])
-def test_automatic_choice_for_ragged_int32_rows(wbits, xbits, M, N, K, warp):
-    """Rows of N % 4 != 0 integers stay on the warp-level kernel below the device-filling size (4096 x 4097 x 1024 is above)."""
+                                                    (2, 2, 2485, 7156, 512, False), (1, 3, 1612, 5888, 256, False), (1, 2, 4096, 4097, 1024, False),
+                                                    (1, 3, 1024, 512, 2048, True), (1, 3, 2048, 2048, 512, False)])
+def test_automatic_choice_for_int32_rows(wbits, xbits, M, N, K, warp):
+    """Rows of N % 4 != 0 integers stay on the warp-level kernel below the device-filling size (4096 x 4097 x 1024 is above),
+    other mid-size problems where it was timed faster."""
     L = _cabi.lib()
     buf = (ctypes.c_uint32 * 64)()
     base = ctypes.addressof(buf)
