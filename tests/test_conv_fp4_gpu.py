@@ -239,3 +239,37 @@ def test_wide_maps_from_planes(cuda_device, H, Wd, CIN, COUT):
     T = oracle.fold_bn(np.ones(COUT, np.float32), np.zeros(COUT, np.float32), float(v.mean()), float(v.std()) / 4, 2)
     got = ap.apconv(to_dev(Wt), to_dev(X), algo="tcgen05", workspace=ws, epilogue=ap.make_epilogue("thresholds", 2, signed="w", thresholds=to_dev(T)))
     assert np.array_equal(to_host(got), oracle.requant_pack(v, 2, 2, T))
+
+
+@pytest.mark.parametrize("B,H,Wd,CIN,COUT,R,stride,mode,pool", [
+    (3, 8, 12, 64, 96, 3, 1, "thresholds", "max"), (2, 16, 16, 128, 160, 3, 2, "lowbits", "max"), (2, 12, 8, 128, 64, 1, 1, "thresholds", "avg"),
+    (1, 8, 8, 1024, 256, 3, 1, "thresholds", "none"),       # few tiles, 72 K blocks: split K
+    (3, 14, 18, 64, 192, 5, 1, "thresholds", "none"), (2, 9, 11, 128, 96, 5, 1, "lowbits", "none"),
+    (100, 14, 14, 256, 256, 3, 1, "thresholds", "none"),    # more than one wave of tile pairs: CTA pairs
+])
+def test_int8_layer_forms_write_nibble_rows(cuda_device, B, H, Wd, CIN, COUT, R, stride, mode, pool):
+    """apnn_conv2d_i8_to_fp4 in the forms of the int8 kernel beside the plain one."""
+    import apnn_tc_b200 as ap
+    from apnn_tc_b200 import _cabi
+    from apnn_tc_b200.ops import _stream_ptr
+    rng = np.random.default_rng(CIN + R + H)
+    p, halo = (R - 1) // 2, 2
+    xl = np.zeros((B, H + 2 * p, Wd + 2 * p, CIN), dtype=np.uint32)
+    xl[:, p:p + H, p:p + Wd] = rng.integers(0, 4, size=(B, H, Wd, CIN))
+    wl = rng.integers(0, 2, size=(COUT, R, R, CIN), dtype=np.uint32)
+    X, Wt = oracle.pack_levels(xl, 2), oracle.pack_levels(wl, 1)
+    v = oracle.signed_correct(oracle.conv_popc(Wt, X, stride=stride, threads=8), oracle.conv_window_sums(X, R, stride), 0)
+    if pool != "none":
+        v = oracle.pool2x2(v, 2 if pool == "max" else 1)
+    T = oracle.fold_bn(np.ones(COUT, np.float32), np.zeros(COUT, np.float32), float(v.mean()), float(v.std()) / 4, 2)
+    want_lv = oracle.levels(v, 2, 2 if mode == "thresholds" else 1, T)
+    epi = ap.make_epilogue(mode, 2, thresholds=to_dev(T), out_halo=halo, out_i8=_cabi.ROWS_FP4, pool=pool)
+    x8 = torch.from_numpy(spread_bytes(xl)).cuda()
+    w8 = torch.from_numpy(spread_bytes((2 * wl.astype(np.int64) - 1).astype(np.uint8).reshape(COUT, -1))).cuda()
+    out = torch.full((B, v.shape[1] + 2 * halo, v.shape[2] + 2 * halo, COUT // 2), 0xEE, dtype=torch.uint8, device="cuda")
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _cabi.check(_cabi.lib().apnn_conv2d_i8_to_fp4(_stream_ptr(), w8.data_ptr(), x8.data_ptr(), out.data_ptr(), B, H, Wd, CIN, COUT, R, stride,
+                                                  1, ctypes.byref(epi), flag.data_ptr()))
+    want = np.full(out.shape, 0xEE, dtype=np.uint8)
+    want[:, halo:-halo, halo:-halo] = spread_nibbles(want_lv)
+    assert np.array_equal(out.cpu().numpy(), want) and int(flag.item()) == 0

@@ -87,3 +87,31 @@ def test_automatic_choice_with_a_workspace_at_any_offset(cuda_device, offset, M,
         assert np.array_equal(to_host(got, np.int32), v)
     else:
         assert np.array_equal(to_host(got), oracle.requant_pack(v, 2, 1, None))
+
+
+# problems on both sides of the automatic choice: one launch from the planes, the warp-level kernel, the expand pass
+@pytest.mark.parametrize("M,N,K", [(64, 1024, 1024), (64, 1024, 8192), (512, 512, 4096), (1024, 1024, 512), (300, 2304, 1024), (2048, 2048, 256),
+                                   (700, 1066, 2816), (96, 64, 16384)])
+@pytest.mark.parametrize("wb,xb,sign", [(1, 1, "x"), (1, 2, "w"), (2, 1, "x"), (2, 2, "none")])
+def test_automatic_choice(cuda_device, M, N, K, wb, xb, sign):
+    import apnn_tc_b200 as ap
+    rng = np.random.default_rng(M + 3 * N + K)
+    W, _ = oracle.value_planes(rng, M, K, wb)
+    X, _ = oracle.value_planes(rng, N, K, xb)
+    v = oracle.gemm_popc(W, X, threads=8)
+    if sign == "w":
+        v = oracle.signed_correct(v, oracle.row_sums(X), 1)
+    elif sign == "x":
+        v = oracle.signed_correct(v, oracle.row_sums(W), 0)
+    Wd, Xd = to_dev(W), to_dev(X)
+    ws = torch.full((ap.gemm_workspace_bytes(M, N, K),), 0xEE, dtype=torch.uint8, device="cuda")
+    got = ap.apmm(Wd, Xd, workspace=ws, epilogue=ap.make_epilogue("int32", signed=sign))
+    ap.gemm_check(ws, M, N, K)
+    assert np.array_equal(to_host(got, np.int32), v)
+    if N % 32:
+        return
+    T = np.sort(rng.integers(int(v.min()) - 1, int(v.max()) + 2, size=(N, 3)), axis=1).astype(np.int32)
+    for mode, bits in (("thresholds", 2), ("lowbits", 3)):
+        got = ap.apmm(Wd, Xd, workspace=ws, epilogue=ap.make_epilogue(mode, bits, signed=sign, thresholds=to_dev(T)))
+        ap.gemm_check(ws, M, N, K)
+        assert np.array_equal(to_host(got), oracle.requant_pack(v, bits, 2 if mode == "thresholds" else 1, T))
