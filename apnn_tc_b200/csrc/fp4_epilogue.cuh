@@ -4,6 +4,7 @@
 #include <cstdint>
 
 #include "apnn_device.cuh"
+#include "tc5_common.cuh"
 
 namespace apnn {
 namespace fp4 {
@@ -37,15 +38,6 @@ struct Fp4Params {
   int* error_flag;
 };
 
-// floor(n / d) == (n * magic) >> shift for every 0 <= n < 2^31 (d >= 1): with L = ceil(log2 d),
-// magic = floor(2^(31+L) / d) + 1 and shift = 31 + L; magic <= 2^32, the product stays below 2^63.
-inline void division_magic(int d, unsigned long long* magic, int* shift) {
-  int L = 0;
-  while ((1ll << L) < d) L++;
-  *shift = 31 + L;
-  *magic = ((1ull << (31 + L)) / (unsigned long long)d) + 1ull;
-}
-
 // B images of H x W output positions inside Hp x Wp stored ones.
 inline void set_image(Fp4Params& p, int B, int H, int W, int Hp, int Wp) {
   p.Bn = B;
@@ -53,8 +45,8 @@ inline void set_image(Fp4Params& p, int B, int H, int W, int Hp, int Wp) {
   p.Wo = W;
   p.wp = Wp;
   p.hpwp = Hp * Wp;
-  division_magic(p.hpwp, &p.magic_hpwp, &p.shift_hpwp);
-  division_magic(p.wp, &p.magic_wp, &p.shift_wp);
+  tc5::division_magic(p.hpwp, &p.magic_hpwp, &p.shift_hpwp);
+  tc5::division_magic(p.wp, &p.magic_wp, &p.shift_wp);
 }
 
 __device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -67,10 +59,6 @@ __device__ __forceinline__ void add_shared_v4(uint32_t* v, uint32_t addr) {
   v[1] = __float_as_uint(__uint_as_float(v[1]) + __uint_as_float(y));
   v[2] = __float_as_uint(__uint_as_float(v[2]) + __uint_as_float(z));
   v[3] = __float_as_uint(__uint_as_float(v[3]) + __uint_as_float(w));
-}
-// eight 32-bit columns of this warp's 32 TMEM lanes <- one value
-__device__ __forceinline__ void tmem_fill8(uint32_t taddr, uint32_t v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(v) : "memory");
 }
 
 // 32 x 32 bit transposition over the warp: bit b of lane a <-> bit a of lane b.
@@ -201,183 +189,183 @@ template <int EPI, class Reload>
 __device__ __forceinline__ void finish_chunk(const Fp4Params& p, uint32_t (&v)[32], const PixelRow& px, int lane, int ch0,
                                              const ChannelThresholds& thr, int nl, int* rows_s, Reload&& reload) {
   const int ch = ch0 + lane;
-            if constexpr (EPI != 0) {
-              if constexpr (EPI == 2) {
-                // accesses are 32 consecutive channels of one pixel; the 32 pixels' rows come from shared memory.  Integers
-                // become floats, and back, through the low mantissa bits of 1.5 * 2^23.
-                __syncwarp();
-                rows_s[32 + lane] = px.dense;
-                __syncwarp();
-                const int4* row4 = reinterpret_cast<const int4*>(rows_s) + 8;
-                constexpr float MAGIC = 12582912.0f;   // 1.5 * 2^23
-                if (ch < p.N && p.residual_in != nullptr) {
-                  const int16_t* R = reinterpret_cast<const int16_t*>(p.residual_in) + ch;
-                  auto add = [&](uint32_t& x, int r) {
-                    x = __float_as_uint(__uint_as_float(x) + (__int_as_float(0x4B400000 + r) - MAGIC));
-                  };
+  if constexpr (EPI != 0) {
+    if constexpr (EPI == 2) {
+      // accesses are 32 consecutive channels of one pixel; the 32 pixels' rows come from shared memory.  Integers
+      // become floats, and back, through the low mantissa bits of 1.5 * 2^23.
+      __syncwarp();
+      rows_s[32 + lane] = px.dense;
+      __syncwarp();
+      const int4* row4 = reinterpret_cast<const int4*>(rows_s) + 8;
+      constexpr float MAGIC = 12582912.0f;   // 1.5 * 2^23
+      if (ch < p.N && p.residual_in != nullptr) {
+        const int16_t* R = reinterpret_cast<const int16_t*>(p.residual_in) + ch;
+        auto add = [&](uint32_t& x, int r) {
+          x = __float_as_uint(__uint_as_float(x) + (__int_as_float(0x4B400000 + r) - MAGIC));
+        };
 #pragma unroll
-                  for (int g = 0; g < 8; g++) {
-                    const int4 d = row4[g];
-                    add(v[4 * g], ld_row16(R, d.x, p.N));
-                    add(v[4 * g + 1], ld_row16(R, d.y, p.N));
-                    add(v[4 * g + 2], ld_row16(R, d.z, p.N));
-                    add(v[4 * g + 3], ld_row16(R, d.w, p.N));
-                  }
-                }
-                if (ch < p.N && p.residual_out != nullptr) {
-                  int16_t* R = reinterpret_cast<int16_t*>(p.residual_out) + ch;
-                  auto sat = [](uint32_t x) {
-                    return __float_as_uint(fminf(fmaxf(__uint_as_float(x), -32768.0f), 32767.0f) + MAGIC);
-                  };
+        for (int g = 0; g < 8; g++) {
+          const int4 d = row4[g];
+          add(v[4 * g], ld_row16(R, d.x, p.N));
+          add(v[4 * g + 1], ld_row16(R, d.y, p.N));
+          add(v[4 * g + 2], ld_row16(R, d.z, p.N));
+          add(v[4 * g + 3], ld_row16(R, d.w, p.N));
+        }
+      }
+      if (ch < p.N && p.residual_out != nullptr) {
+        int16_t* R = reinterpret_cast<int16_t*>(p.residual_out) + ch;
+        auto sat = [](uint32_t x) {
+          return __float_as_uint(fminf(fmaxf(__uint_as_float(x), -32768.0f), 32767.0f) + MAGIC);
+        };
 #pragma unroll
-                  for (int g = 0; g < 8; g++) {
-                    const int4 d = row4[g];
-                    st_row16(R, d.x, p.N, sat(v[4 * g]));
-                    st_row16(R, d.y, p.N, sat(v[4 * g + 1]));
-                    st_row16(R, d.z, p.N, sat(v[4 * g + 2]));
-                    st_row16(R, d.w, p.N, sat(v[4 * g + 3]));
-                  }
-                }
-              }
-              const uint32_t b1 = below_bits(v, thr.nt1), b2 = below_bits(v, thr.nt2), b3 = below_bits(v, thr.nt3);
-              reload();   // in flight during the rest of this chunk
-              // level = number of thresholds reached, as two bit words; then one word pair per pixel
-              const uint32_t p0 = __brev(transpose_bits(~(b1 ^ b2 ^ b3), lane));
-              const uint32_t p1 = __brev(transpose_bits(~((b1 & b2) | (b1 & b3) | (b2 & b3)), lane));
-              if (px.row >= 0) {
-                if (p.rows_out == 2) {
-                  *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + (((long long)px.row * p.N + ch0) >> 1)) = nibbles_of(p0, p1);
-                } else if (p.rows_out == 1) {
-                  uint32_t r[8];
+        for (int g = 0; g < 8; g++) {
+          const int4 d = row4[g];
+          st_row16(R, d.x, p.N, sat(v[4 * g]));
+          st_row16(R, d.y, p.N, sat(v[4 * g + 1]));
+          st_row16(R, d.z, p.N, sat(v[4 * g + 2]));
+          st_row16(R, d.w, p.N, sat(v[4 * g + 3]));
+        }
+      }
+    }
+    const uint32_t b1 = below_bits(v, thr.nt1), b2 = below_bits(v, thr.nt2), b3 = below_bits(v, thr.nt3);
+    reload();   // in flight during the rest of this chunk
+    // level = number of thresholds reached, as two bit words; then one word pair per pixel
+    const uint32_t p0 = __brev(transpose_bits(~(b1 ^ b2 ^ b3), lane));
+    const uint32_t p1 = __brev(transpose_bits(~((b1 & b2) | (b1 & b3) | (b2 & b3)), lane));
+    if (px.row >= 0) {
+      if (p.rows_out == 2) {
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + (((long long)px.row * p.N + ch0) >> 1)) = nibbles_of(p0, p1);
+      } else if (p.rows_out == 1) {
+        uint32_t r[8];
 #pragma unroll
-                  for (int q = 0; q < 8; q++) r[q] = ((p0 >> q) & 0x01010101u) | (((p1 >> q) & 0x01010101u) << 1);
-                  store_32(reinterpret_cast<uint8_t*>(p.out) + (long long)px.row * p.N + ch0, r);
-                } else {
-                  uint32_t* O = reinterpret_cast<uint32_t*>(p.out) + (long long)px.row * (p.N >> 5) + (ch0 >> 5);
-                  O[0] = p0;
-                  if (p.out_bits > 1) O[p.out_plane_words] = p1;
-                }
-              }
-              __syncwarp();
-            } else {
-              const bool ch_ok = ch < p.N;
+        for (int q = 0; q < 8; q++) r[q] = ((p0 >> q) & 0x01010101u) | (((p1 >> q) & 0x01010101u) << 1);
+        store_32(reinterpret_cast<uint8_t*>(p.out) + (long long)px.row * p.N + ch0, r);
+      } else {
+        uint32_t* O = reinterpret_cast<uint32_t*>(p.out) + (long long)px.row * (p.N >> 5) + (ch0 >> 5);
+        O[0] = p0;
+        if (p.out_bits > 1) O[p.out_plane_words] = p1;
+      }
+    }
+    __syncwarp();
+  } else {
+    const bool ch_ok = ch < p.N;
 #pragma unroll
-              for (int j = 0; j < 32; j++) v[j] = (uint32_t)__float2int_rn(__uint_as_float(v[j]));
-              // every access below is 32 consecutive channels of one pixel; the 32 pixels' rows come from shared memory
-              __syncwarp();
-              rows_s[lane] = px.row;
-              rows_s[32 + lane] = px.dense;
-              __syncwarp();
-              const int4* row4 = reinterpret_cast<const int4*>(rows_s);
-              if (ch_ok && p.residual_in != nullptr) {
-                if (p.res16_in) {
-                  const int16_t* R = reinterpret_cast<const int16_t*>(p.residual_in) + ch;
+    for (int j = 0; j < 32; j++) v[j] = (uint32_t)__float2int_rn(__uint_as_float(v[j]));
+    // every access below is 32 consecutive channels of one pixel; the 32 pixels' rows come from shared memory
+    __syncwarp();
+    rows_s[lane] = px.row;
+    rows_s[32 + lane] = px.dense;
+    __syncwarp();
+    const int4* row4 = reinterpret_cast<const int4*>(rows_s);
+    if (ch_ok && p.residual_in != nullptr) {
+      if (p.res16_in) {
+        const int16_t* R = reinterpret_cast<const int16_t*>(p.residual_in) + ch;
 #pragma unroll
-                  for (int g = 0; g < 8; g++) {
-                    const int4 d = row4[8 + g];
-                    v[4 * g] += (uint32_t)ld_row16(R, d.x, p.N);
-                    v[4 * g + 1] += (uint32_t)ld_row16(R, d.y, p.N);
-                    v[4 * g + 2] += (uint32_t)ld_row16(R, d.z, p.N);
-                    v[4 * g + 3] += (uint32_t)ld_row16(R, d.w, p.N);
-                  }
-                } else {
-                  const int32_t* R = p.residual_in + ch;
+        for (int g = 0; g < 8; g++) {
+          const int4 d = row4[8 + g];
+          v[4 * g] += (uint32_t)ld_row16(R, d.x, p.N);
+          v[4 * g + 1] += (uint32_t)ld_row16(R, d.y, p.N);
+          v[4 * g + 2] += (uint32_t)ld_row16(R, d.z, p.N);
+          v[4 * g + 3] += (uint32_t)ld_row16(R, d.w, p.N);
+        }
+      } else {
+        const int32_t* R = p.residual_in + ch;
 #pragma unroll
-                  for (int g = 0; g < 8; g++) {
-                    const int4 d = row4[8 + g];
-                    v[4 * g] += (uint32_t)ld_row32(R, d.x, p.N);
-                    v[4 * g + 1] += (uint32_t)ld_row32(R, d.y, p.N);
-                    v[4 * g + 2] += (uint32_t)ld_row32(R, d.z, p.N);
-                    v[4 * g + 3] += (uint32_t)ld_row32(R, d.w, p.N);
-                  }
-                }
-              }
-              if (ch_ok && p.residual_out != nullptr) {
-                if (p.res16_out) {
-                  int16_t* R = reinterpret_cast<int16_t*>(p.residual_out) + ch;
-                  auto sat = [](uint32_t x) { return (uint32_t)min(max((int)x, -32768), 32767); };
+        for (int g = 0; g < 8; g++) {
+          const int4 d = row4[8 + g];
+          v[4 * g] += (uint32_t)ld_row32(R, d.x, p.N);
+          v[4 * g + 1] += (uint32_t)ld_row32(R, d.y, p.N);
+          v[4 * g + 2] += (uint32_t)ld_row32(R, d.z, p.N);
+          v[4 * g + 3] += (uint32_t)ld_row32(R, d.w, p.N);
+        }
+      }
+    }
+    if (ch_ok && p.residual_out != nullptr) {
+      if (p.res16_out) {
+        int16_t* R = reinterpret_cast<int16_t*>(p.residual_out) + ch;
+        auto sat = [](uint32_t x) { return (uint32_t)min(max((int)x, -32768), 32767); };
 #pragma unroll
-                  for (int g = 0; g < 8; g++) {
-                    const int4 d = row4[8 + g];
-                    st_row16(R, d.x, p.N, sat(v[4 * g]));
-                    st_row16(R, d.y, p.N, sat(v[4 * g + 1]));
-                    st_row16(R, d.z, p.N, sat(v[4 * g + 2]));
-                    st_row16(R, d.w, p.N, sat(v[4 * g + 3]));
-                  }
-                } else {
-                  int32_t* R = p.residual_out + ch;
+        for (int g = 0; g < 8; g++) {
+          const int4 d = row4[8 + g];
+          st_row16(R, d.x, p.N, sat(v[4 * g]));
+          st_row16(R, d.y, p.N, sat(v[4 * g + 1]));
+          st_row16(R, d.z, p.N, sat(v[4 * g + 2]));
+          st_row16(R, d.w, p.N, sat(v[4 * g + 3]));
+        }
+      } else {
+        int32_t* R = p.residual_out + ch;
 #pragma unroll
-                  for (int g = 0; g < 8; g++) {
-                    const int4 d = row4[8 + g];
-                    st_row32(R, d.x, p.N, v[4 * g]);
-                    st_row32(R, d.y, p.N, v[4 * g + 1]);
-                    st_row32(R, d.z, p.N, v[4 * g + 2]);
-                    st_row32(R, d.w, p.N, v[4 * g + 3]);
-                  }
-                }
-              }
-              if (p.out_mode == OUT_FLOAT) {
-                // two separately rounded operations per element (the CPU check computes the same two)
-                const float sc = ch_ok ? __ldg(p.affine_scale + ch) : 0.0f, bi = ch_ok ? __ldg(p.affine_bias + ch) : 0.0f;
+        for (int g = 0; g < 8; g++) {
+          const int4 d = row4[8 + g];
+          st_row32(R, d.x, p.N, v[4 * g]);
+          st_row32(R, d.y, p.N, v[4 * g + 1]);
+          st_row32(R, d.z, p.N, v[4 * g + 2]);
+          st_row32(R, d.w, p.N, v[4 * g + 3]);
+        }
+      }
+    }
+    if (p.out_mode == OUT_FLOAT) {
+      // two separately rounded operations per element (the CPU check computes the same two)
+      const float sc = ch_ok ? __ldg(p.affine_scale + ch) : 0.0f, bi = ch_ok ? __ldg(p.affine_bias + ch) : 0.0f;
 #pragma unroll
-                for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__fadd_rn(__fmul_rn((float)(int)v[j], sc), bi));
-              }
-              if (p.out_mode == OUT_INT32 || p.out_mode == OUT_FLOAT) {
-                int32_t* D = reinterpret_cast<int32_t*>(p.out) + ch;
-                if (ch_ok) {
+      for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__fadd_rn(__fmul_rn((float)(int)v[j], sc), bi));
+    }
+    if (p.out_mode == OUT_INT32 || p.out_mode == OUT_FLOAT) {
+      int32_t* D = reinterpret_cast<int32_t*>(p.out) + ch;
+      if (ch_ok) {
 #pragma unroll
-                  for (int g = 0; g < 8; g++) {
-                    const int4 d = row4[g];
-                    st_row32(D, d.x, p.N, v[4 * g]);
-                    st_row32(D, d.y, p.N, v[4 * g + 1]);
-                    st_row32(D, d.z, p.N, v[4 * g + 2]);
-                    st_row32(D, d.w, p.N, v[4 * g + 3]);
-                  }
-                }
-              } else {
-                // packed modes need N % 32 == 0: all 32 channels of the warp exist
-                if (p.out_mode == OUT_THRESHOLDS) {
-                  uint32_t lv[32];
+        for (int g = 0; g < 8; g++) {
+          const int4 d = row4[g];
+          st_row32(D, d.x, p.N, v[4 * g]);
+          st_row32(D, d.y, p.N, v[4 * g + 1]);
+          st_row32(D, d.z, p.N, v[4 * g + 2]);
+          st_row32(D, d.w, p.N, v[4 * g + 3]);
+        }
+      }
+    } else {
+      // packed modes need N % 32 == 0: all 32 channels of the warp exist
+      if (p.out_mode == OUT_THRESHOLDS) {
+        uint32_t lv[32];
 #pragma unroll
-                  for (int j = 0; j < 32; j++) lv[j] = 0u;
-                  const int32_t* T = p.thresholds + (long long)ch * nl;
+        for (int j = 0; j < 32; j++) lv[j] = 0u;
+        const int32_t* T = p.thresholds + (long long)ch * nl;
 #pragma unroll 1
-                  for (int t = 0; t < nl; t++) {
-                    const int thr = __ldg(T + t);
+        for (int t = 0; t < nl; t++) {
+          const int thr = __ldg(T + t);
 #pragma unroll
-                    for (int j = 0; j < 32; j++) lv[j] += ((int)v[j] >= thr) ? 1u : 0u;
-                  }
+          for (int j = 0; j < 32; j++) lv[j] += ((int)v[j] >= thr) ? 1u : 0u;
+        }
 #pragma unroll
-                  for (int j = 0; j < 32; j++) v[j] = lv[j];
-                }
-                uint32_t r[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-                uint32_t first = 0u, second = 0u;
+        for (int j = 0; j < 32; j++) v[j] = lv[j];
+      }
+      uint32_t r[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      uint32_t first = 0u, second = 0u;
 #pragma unroll 1
-                for (int b = 0; b < p.out_bits; b++) {
-                  uint32_t w = 0u;
+      for (int b = 0; b < p.out_bits; b++) {
+        uint32_t w = 0u;
 #pragma unroll
-                  for (int j = 0; j < 32; j++) w |= ((v[j] >> b) & 1u) << j;
-                  const uint32_t plane = __brev(transpose_bits(w, lane));
-                  if (p.rows_out == 1) {
+        for (int j = 0; j < 32; j++) w |= ((v[j] >> b) & 1u) << j;
+        const uint32_t plane = __brev(transpose_bits(w, lane));
+        if (p.rows_out == 1) {
 #pragma unroll
-                    for (int q = 0; q < 8; q++) r[q] |= ((plane >> q) & 0x01010101u) << b;
-                  } else if (p.rows_out == 2) {
-                    if (b == 0) first = plane;
-                    else second = plane;
-                  } else if (px.row >= 0) {
-                    reinterpret_cast<uint32_t*>(p.out)[b * p.out_plane_words + (long long)px.row * (p.N >> 5) + (ch0 >> 5)] = plane;
-                  }
-                }
-                if (px.row >= 0) {
-                  if (p.rows_out == 1) store_32(reinterpret_cast<uint8_t*>(p.out) + (long long)px.row * p.N + ch0, r);
-                  else if (p.rows_out == 2)
-                    *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + (((long long)px.row * p.N + ch0) >> 1)) =
-                        nibbles_of(first, second);
-                }
-              }
-              __syncwarp();   // lanes that skipped a store rejoin before the warp-wide TMEM load
-              reload();
-            }
+          for (int q = 0; q < 8; q++) r[q] |= ((plane >> q) & 0x01010101u) << b;
+        } else if (p.rows_out == 2) {
+          if (b == 0) first = plane;
+          else second = plane;
+        } else if (px.row >= 0) {
+          reinterpret_cast<uint32_t*>(p.out)[b * p.out_plane_words + (long long)px.row * (p.N >> 5) + (ch0 >> 5)] = plane;
+        }
+      }
+      if (px.row >= 0) {
+        if (p.rows_out == 1) store_32(reinterpret_cast<uint8_t*>(p.out) + (long long)px.row * p.N + ch0, r);
+        else if (p.rows_out == 2)
+          *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(p.out) + (((long long)px.row * p.N + ch0) >> 1)) =
+              nibbles_of(first, second);
+      }
+    }
+    __syncwarp();   // lanes that skipped a store rejoin before the warp-wide TMEM load
+    reload();
+  }
 }
 
 }  // namespace fp4

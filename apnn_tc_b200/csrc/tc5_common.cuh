@@ -5,6 +5,7 @@
 
 #include <cstdint>
 
+#include "api_internal.h"
 #include "apnn_device.cuh"
 
 namespace apnn {
@@ -122,6 +123,51 @@ __device__ __forceinline__ uint64_t make_smem_desc_k(uint32_t saddr) {
   d |= (uint64_t)1 << 46;
   d |= (uint64_t)(BKB == 128 ? 2 : 4) << 61;
   return d;
+}
+
+// ------------------------------------------------------------------ clusters and CTA pairs
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// Cluster-wide barrier with release / acquire semantics (all threads of all CTAs of the cluster).
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared::cluster address of the same location in CTA `rank` of this cluster
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+// TMA tile load of a CTA pair: data lands in this CTA, the bytes complete on `bar_cluster`
+// (a shared::cluster address, here always the leader's barrier)
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar_cluster) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+      "[%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar_cluster)
+      : "memory");
+}
+// eight 32-bit columns of this warp's 32 TMEM lanes <- one value
+__device__ __forceinline__ void tmem_fill8(uint32_t taddr, uint32_t v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(v) : "memory");
+}
+
+// ------------------------------------------------------------------ host side
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline EncodeTiledFn encode_tiled_fn() { return reinterpret_cast<EncodeTiledFn>(tensor_map_encoder()); }
+
+// floor(n / d) == (n * magic) >> shift for every 0 <= n < 2^31 (d >= 1): with L = ceil(log2 d),
+// magic = floor(2^(31+L) / d) + 1 and shift = 31 + L; magic <= 2^32, the product stays below 2^63.
+inline void division_magic(int d, unsigned long long* magic, int* shift) {
+  int L = 0;
+  while ((1ll << L) < d) L++;
+  *shift = 31 + L;
+  *magic = ((1ull << (31 + L)) / (unsigned long long)d) + 1ull;
 }
 
 }  // namespace tc5

@@ -26,7 +26,6 @@
 // tmem_empty in the leader (every epilogue warp of both CTAs).  All waits are time-bounded.  The loads carry no cluster multicast.
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 
 #include "api_internal.h"
 #include "fp4_epilogue.cuh"
@@ -54,32 +53,11 @@ constexpr int BAR_BYTES = 512;
 constexpr int ROWS_BYTES = epi_warps(0, 64) * 64 * 4;   // per epilogue warp: the output rows of a chunk's 32 pixels
 constexpr int SMEM_LIMIT = 232448;
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
 // Arrival that says "this warp's TMEM loads are complete" (they are: tcgen05.wait::ld has returned).  Nothing else is
 // published by it, so it is relaxed: a release at cluster scope waits for every output store the warp has in flight
 // (128 x 56x56, 256 -> 256 channels: 95 -> 86 us).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// TMA tile load of a CTA pair: data lands in this CTA, the bytes complete on the leader's barrier
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar_cluster) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-      "[%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar_cluster)
-      : "memory");
 }
 // pair_mask: the two CTAs of this pair as bits of the cluster rank
 __device__ __forceinline__ void tc_commit_pair(uint32_t bar, uint16_t pair_mask) {
@@ -355,13 +333,9 @@ tc5_conv_fp4_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // byte rows [rows][pitch], boxes of span bytes x box_rows rows, swizzle span = span (128 or 64)
 bool make_rows_map(CUtensorMap* map, const void* base, long long rows, long long pitch, int box_rows, int span) {
-  EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(tensor_map_encoder());
+  EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return false;
   cuuint64_t dims[2] = {(cuuint64_t)pitch, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)pitch};
@@ -393,11 +367,12 @@ Fp4Plan plan_np(long long flat_rows, int COUT, int R, int Wp, int kbytes_per_tap
   const int pairs = sms / 2;
   for (int splits = 1; splits <= 4 && splits * 2 <= cblocks + (splits == 1 ? 1 : 0); splits *= 2) {
     Fp4Plan here = {0, splits, 0, 0};
+    const int resident = splits > 1 ? fp4_cluster_capacity(splits, span) : 0;
     for (int np = MAX_NP; np >= 32; np -= 32) {
       const int rows = box_rows_of(R, Wp, np);
       if (rows > 256) continue;
       const long long tiles = ((flat_rows + np - 1) / np) * tiles_n;
-      if (splits > 1 && (tiles * splits > pairs || tiles > fp4_cluster_capacity(splits, span))) continue;
+      if (splits > 1 && (tiles * splits > pairs || tiles > resident)) continue;
       const long long waves = (tiles + pairs - 1) / pairs;
       const long long kb = (cblocks + splits - 1) / splits;   // K blocks of one pair
       const long long mma = kb * R * R * np * 2 * span / 128;
@@ -466,38 +441,11 @@ cudaError_t launch_fp4(cudaStream_t s, const CUtensorMap& map_x, const CUtensorM
   return cudaLaunchKernelEx(&cfg, tc5_conv_fp4_kernel<RR, BKB, EPI, SPLIT>, map_x, map_w, p);
 }
 
-// How many clusters of `splits` pairs the device holds at once (0 on error); cached per device.
+// How many clusters of `splits` pairs the device holds at once.
 int fp4_cluster_capacity(int splits, int span) {
-  static std::mutex mu;
-  static int cache[16][2][2] = {};   // value + 1
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 16 || (splits != 2 && splits != 4)) return 0;
-  std::lock_guard<std::mutex> lock(mu);
-  int& slot = cache[dev][splits == 4][span == 64];
-  if (slot) return slot - 1;
   const void* kernel = span == 128 ? reinterpret_cast<const void*>(tc5_conv_fp4_kernel<1, 128, 1, true>)
                                    : reinterpret_cast<const void*>(tc5_conv_fp4_kernel<1, 64, 1, true>);
-  int n = 0;
-  if (ensure_max_smem(kernel, SMEM_LIMIT) == cudaSuccess) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(2 * splits * device_sm_count()), 1, 1);
-    cfg.blockDim = dim3(threads_of(1, span), 1, 1);
-    cfg.dynamicSmemBytes = SMEM_LIMIT;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)(2 * splits);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-  }
-  slot = n + 1;
-  return n;
+  return cluster_capacity(kernel, threads_of(1, span), SMEM_LIMIT, 2 * splits);
 }
 
 template <int RR, int SPAN>

@@ -35,7 +35,6 @@
 
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 
 #include "api_internal.h"
 #include "apnn_device.cuh"
@@ -267,22 +266,6 @@ __device__ __forceinline__ void tile_coords(int tile, int tiles_m, int tiles_n, 
   tn = r / rows;
 }
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// Cluster-wide barrier with release / acquire semantics (all threads of all CTAs of the cluster).
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared::cluster address of the same location in CTA `rank` of this cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
 // ---- CTA pairs (cta_group::2).  PAIR = true: the even CTA of a pair (the leader) issues every MMA over 256 rows
 // (its own 128-row A tile and the peer's) and both halves of the B tile; TMA loads of both CTAs complete on the
 // leader's barrier; the leader's commits arrive on the barrier at the same offset in both CTAs.
@@ -1195,12 +1178,6 @@ tc5_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #undef KB_LAST
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled_fn() { return reinterpret_cast<EncodeTiledFn>(tensor_map_encoder()); }
-
 // rows x K bytes, row-major; box = box_rows x span bytes (span = 128 or 64 = the swizzle span), zero fill outside
 bool make_operand_map(CUtensorMap* map, const void* base, long long rows, long long K, int box_rows, int span = 128) {
   EncodeTiledFn fn = encode_tiled_fn();
@@ -1234,15 +1211,6 @@ bool make_activation_map(CUtensorMap* map, const void* base, int B, int Hp, int 
 }
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
-
-// floor(n / d) == (n * magic) >> shift for every 0 <= n < 2^31 (d >= 1): with L = ceil(log2 d),
-// magic = floor(2^(31+L) / d) + 1 and shift = 31 + L; magic <= 2^32, the product stays below 2^63.
-void division_magic(int d, unsigned long long* magic, int* shift) {
-  int L = 0;
-  while ((1ll << L) < d) L++;
-  *shift = 31 + L;
-  *magic = ((1ull << (31 + L)) / (unsigned long long)d) + 1ull;
-}
 
 // Shared-memory plan: keep the whole B operand resident when the problem has one tile column
 // and its K blocks leave room for at least three A stages; otherwise a ring of A+B stages.
@@ -1404,40 +1372,12 @@ int pick_bn(long long tiles_m, int N, int sms) {
   return w128 < w256 ? 128 : 256;
 }
 
-// How many clusters of `ctas` CTAs of the split-K kernel (single-CTA or CTA-pair form) the device holds at once
-// (0 on error); cached.
-int cluster_capacity(int bn, bool pair, int ctas) {
-  static std::mutex mu;
-  static int cache[16][3][4] = {};   // [device][128 / 256 / 256 pair][log2 ctas], value + 1
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 16 || ctas < 2 || ctas > 8) return 0;
-  const int li = ctas == 2 ? 1 : ctas == 4 ? 2 : 3, bi = pair ? 2 : (bn == 256 ? 1 : 0);
-  std::lock_guard<std::mutex> lock(mu);
-  if (cache[dev][bi][li]) return cache[dev][bi][li] - 1;
+// How many clusters of `ctas` CTAs of the split-K kernel (single-CTA or CTA-pair form) the device holds at once.
+int split_capacity(int bn, bool pair, int ctas) {
   const void* kernel = pair ? reinterpret_cast<const void*>(tc5_gemm_kernel<256, 128, true, 0, true>)
                             : bn == 256 ? reinterpret_cast<const void*>(tc5_gemm_kernel<256, 128, true, 0, false>)
                                         : reinterpret_cast<const void*>(tc5_gemm_kernel<128, 128, true, 0, false>);
-  int n = 0;
-  if (ensure_max_smem(kernel, SMEM_LIMIT) == cudaSuccess) {
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)(ctas * device_sm_count()), 1, 1);
-    cfg.blockDim = dim3(THREADS, 1, 1);
-    cfg.dynamicSmemBytes = SMEM_LIMIT;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      n = 0;
-    }
-  }
-  cache[dev][bi][li] = n + 1;
-  return n;
+  return cluster_capacity(kernel, THREADS, SMEM_LIMIT, ctas);
 }
 
 // Tile plan of one launch: tile width, whether CTA pairs share the B tile, and how many ways K is split over a
@@ -1477,7 +1417,7 @@ TilePlan pick_plan(long long tiles_m, int N, int kblocks, int sms, int bn_plain,
         // 1 - 20 % slower as pairs (batch 8, 16x16 convolutions of 640 - 1024 channels)
         if (cs > 1 && pair && !pair_split) break;
         if (cs > 1 && (no_split || !may_split || kblocks < 8 || cs > cand / 32 || kblocks / cs < 4 || (pair ? 2 : 1) * cs > 8)) break;
-        if (cs > 1 && (units * cs > slots || units > cluster_capacity(cand, pair != 0, (pair ? 2 : 1) * cs))) break;
+        if (cs > 1 && (units * cs > slots || units > split_capacity(cand, pair != 0, (pair ? 2 : 1) * cs))) break;
         const long long cost = waves(units * cs, slots) * ((kblocks + cs - 1) / cs + (cs > 1 ? 4 : 0)) * rows;
         if (cost < best_cost) {
           best_cost = cost;

@@ -18,7 +18,6 @@
 // (128 x 4096 x 9216, thresholds: 13.4 us, 33.5 on the warp-level kernel; 64 x 128 x 128: 3.7 against 7.5).
 #include <cstdlib>
 #include <cstring>
-#include <mutex>
 
 #include "api_internal.h"
 #include "core_launch.h"
@@ -58,20 +57,6 @@ struct PlanesParams {
   uint32_t bars_off;
 };
 
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-  return r;
-}
 __device__ __forceinline__ void tc_mma_mxf4(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sf_tmem,
                                             uint32_t accumulate) {
   asm volatile(
@@ -413,13 +398,9 @@ cudaError_t launch_planes(cudaStream_t s, const CUtensorMap& map_px, const CUten
   return cudaLaunchKernelEx(&cfg, tc5_planes_kernel<PXB, CHB, EPI, SPLIT>, map_px, map_ch, q);
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 // planes [bits][rows][K/8 bytes]; box = 128 bytes x box_rows rows x all planes, 128-byte swizzle, zero fill outside
 bool make_planes_map(CUtensorMap* map, const void* planes, long long rows, int K, int bits, int box_rows) {
-  EncodeTiledFn fn = reinterpret_cast<EncodeTiledFn>(tensor_map_encoder());
+  EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return false;
   const cuuint64_t row = (cuuint64_t)K / 8;
   cuuint64_t dims[3] = {row, (cuuint64_t)rows, (cuuint64_t)bits};
