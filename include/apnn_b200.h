@@ -63,8 +63,10 @@ enum {
   APNN_ALGO_BMMA = 1,    /* 1-bit and-popcount mma.sync per plane pair (emulated on sm_100a;
                             kept as the measured comparison), no workspace */
   APNN_ALGO_IMMA = 2,    /* planes spread to u8 in registers, mma.sync m16n8k32, no workspace */
-  APNN_ALGO_TCGEN05 = 3, /* planes expanded to int8 in the workspace, TMA-fed tcgen05 kind::i8
-                            with TMEM accumulators */
+  APNN_ALGO_TCGEN05 = 3, /* planes expanded in the workspace, TMA-fed tcgen05 with TMEM accumulators:
+                            int8 and kind::i8, or, for operands of at most two bits where that is
+                            the faster path, e2m1 nibbles and kind::mxf4 (the same integers;
+                            APNN_FP4=0 in the environment keeps int8) */
   APNN_ALGO_TCGEN05_PAIR = 4 /* GEMM only: the same on CTA pairs (cta_group::2, 256x256 tiles,
                                 each SM stages half of both operands); same workspace */
 };
@@ -93,7 +95,8 @@ typedef struct apnn_epilogue {
                                  "save_residual" output of NN/param.h:943-945 */
   int32_t n_peer_out;         /* GEMM on the tcgen05 CTA-pair kernel only: number of extra
                                  destinations in peer_out (0..7) */
-  int32_t out_i8;             /* apnn_conv2d_i8 / apnn_gemm_i8 only, with a quantising out_mode: 1 =
+  int32_t out_i8;             /* apnn_conv2d_i8 / apnn_gemm_i8 / apnn_conv2d_fp4 / apnn_linear_fp4 only,
+                                 with a quantising out_mode (APNN_ROWS_FP4, below: e2m1 nibbles): 1 =
                                  write one byte per output element (the level), rows of `channels`
                                  bytes in the byte order of apnn_expand_planes and the same ring
                                  as the packed output, instead of packed planes -- the next
@@ -137,10 +140,13 @@ apnn_status apnn_gemm(void *stream, int wbits, int xbits, const void *W, const v
  * APNN_OUT_LOWBITS it replaces apmm_w1a2_decompose (LIB/66_bmmaTensorCoreGemm.cuh:81-280)
  * and apmm_w2a2_decompose (LIB/73_bmmaTensorCoreGemm.cuh:81-297), which FC_new_global /
  * Output_new_global call (NN/kernel.cuh:299-318).  Packed modes need N % 32 == 0.
- * epi == NULL means int32 output.  workspace may be NULL for every algorithm but APNN_ALGO_TCGEN05.
+ * epi == NULL means int32 output.  workspace may be NULL for every algorithm but APNN_ALGO_TCGEN05,
+ * which needs it 32-byte aligned, as AUTO does where that path is the only one or the problem fills the
+ * device; elsewhere a workspace may lie at any address.
  * With a workspace (APNN_ALGO_TCGEN05, or AUTO) every pair of widths from {1, 2, 3, 4, 8} runs --
  * the reference's w4a4 / w1a8 / w2a8 programs (LIB/83, 77, 76_bmmaTensorCoreGemm.cu) included:
- * on the int8 path a level of up to 8 bits is one byte whatever its width.  apnn_conv2d_ex
+ * on the int8 path a level of up to 8 bits is one byte whatever its width (levels of at most two
+ * bits may run as e2m1 nibbles instead).  apnn_conv2d_ex
  * follows the same rule. */
 apnn_status apnn_gemm_ex(void *stream, int algo, int wbits, int xbits, const void *W,
                          const void *X, void *D, int M, int N, int K,
@@ -193,7 +199,7 @@ apnn_status apnn_gemm_w8(void *stream, const void *W8, int xbits, const void *X,
  * one- or two-plane operand and the -1 / +1 of a signed one-plane operand are e2m1 values; with every block scale
  * factor set to 1 all products and partial sums are small integers, exact in fp32 while |sum| < 2^24.  So for
  * wbits, xbits <= 2 the contraction of apmm_w1a2 / apmm_w2a2 (LIB/71_, 72_bmmaTensorCoreGemm.cu:80) runs there
- * bit for bit (tests compare with the oracle and with the int8 path, sums up to 786432 included).
+ * bit for bit (tests compare with the oracle and with the int8 path, and with a float64 product up to sums of 2^24 - 640).
  * apnn_expand_planes_fp4: planes[bits][rows][K/32] -> out_fp4[rows][K/2], two elements per byte (bits 1 or 2;
  *   is_signed only with bits == 1), K % 256 == 0, a fixed permutation inside each group of 32 k.
  * apnn_gemm_fp4: D = W4 * X4^T over such operands on CTA pairs (256 x 224 tiles), epilogue as apnn_gemm_i8
@@ -248,8 +254,9 @@ apnn_status apnn_conv2d(void *stream, int wbits, int xbits, const void *Wt, cons
                         const apnn_epilogue *epi);
 
 /* apnn_conv2d_ex adds the algorithm / workspace choice.  APNN_ALGO_TCGEN05 (stride 1 or 2, any supported R)
- * expands activations and filter to int8 in the workspace and runs the implicit GEMM on
- * tcgen05 kind::i8, each A tile a 4-D TMA box of output pixels; APNN_ALGO_AUTO picks it when
+ * expands activations and filter in the workspace, in one launch, and runs the implicit GEMM on
+ * tcgen05: int8 and kind::i8, or for operands of at most two bits (R 1 or 3, stride 1, no pooling)
+ * e2m1 nibbles and kind::mxf4 where the estimated time is shorter; APNN_ALGO_AUTO picks it when
  * the workspace is large enough and the contraction is at least ~2 GFLOP, else the
  * warp-level kernel.  apnn_conv2d_check is apnn_gemm_check for this workspace layout.
  * apnn_conv2d_i8 runs on operands already expanded by apnn_expand_planes: X8[B][H+2h][W+2h][CIN]
@@ -272,8 +279,9 @@ apnn_status apnn_conv2d_i8(void *stream, const void *W8, const void *X8, void *O
  * twice the int8 tensor rate, bit for bit the same results.  R is 1 or 3, CIN % 128 == 0, the sums
  * stay below 2^24 (9*R*R*CIN < 2^24), no pooling, no APNN_OUT_FLOAT, and for R = 3 the stored rows are at
  * most 119 pixels wide (the rows the taps of a tile reach must fit one 256-row box), else
- * APNN_ERR_UNSUPPORTED.  Above 100 pixels the box leaves so few pixels per tile that apnn_conv2d_i8 is faster.  epi->out_i8 = 1 writes int8 rows, APNN_ROWS_FP4 nibble rows (out_bits <= 2):
- * the operand of the next such layer.  No reference counterpart. */
+ * APNN_ERR_UNSUPPORTED.  Above 100 pixels the box leaves so few pixels per tile that apnn_conv2d_i8 is faster.
+ * epi->out_i8 = 1 writes int8 rows, APNN_ROWS_FP4 nibble rows (out_bits <= 2): the operand of the next such
+ * layer.  No reference counterpart. */
 #define APNN_ROWS_FP4 2
 apnn_status apnn_conv2d_fp4(void *stream, const void *W4, const void *X4, void *Out, int B, int H, int W,
                             int CIN, int COUT, int R, const apnn_epilogue *epi, int *status_flag);
