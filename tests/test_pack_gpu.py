@@ -207,3 +207,18 @@ def test_pack_groups_of_a_trip(cuda_device, rows, C, bits, source):
     x.reshape(-1)[: min(probe.size, x.size)] = probe[: x.size]
     got = to_host(ap.images_quantization(torch.from_numpy(x).cuda(), bits))
     assert np.array_equal(got, oracle.bit_compress(oracle.quantize(x, bits), bits))
+
+
+@pytest.mark.parametrize("bits", [1, 2, 3, 4, 5, 6, 7, 8])
+@pytest.mark.parametrize("C", [3, 12, 30, 200])
+def test_float_packers_at_every_level_edge(cuda_device, bits, C):
+    """Floats on, one below and one above every rounding edge of every width, in each form of the packers."""
+    import apnn_tc_b200 as ap
+    n = 1 << bits
+    edges = (20.0 * (np.arange(n) + 0.5) / n - 10.0).astype(np.float32)
+    x = np.concatenate([edges] + [np.nextafter(edges, np.float32(s * 20)) for s in (-1, 1)]
+                       + [np.array([-np.inf, np.inf, np.nan, -0.0, 10.0, -10.0, 1e30], np.float32)])
+    x = np.resize(x, ((x.size + C - 1) // C * C,)).reshape(-1, C)
+    want = oracle.bit_compress(oracle.quantize(np.where(np.isnan(x), np.float32(-10), x), bits), bits)
+    got = to_host(ap.images_quantization(torch.from_numpy(x.copy()).cuda(), bits))
+    assert np.array_equal(got, want)
