@@ -1,5 +1,6 @@
 """Kernels launched as programmatic dependents may begin while the previous kernel of their stream still runs, and the
-warp-level kernels let them begin before they have read anything.  So nothing global is written before the dependency wait."""
+warp-level kernels let them begin before they have read anything.  So nothing global is read or written before the dependency
+wait."""
 import glob
 import os
 import re
@@ -12,6 +13,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 WAIT = re.compile(r"grid_dependency_wait\(\)|griddepcontrol\.wait")
 # a store through a pointer parameter, a global store instruction, an atomic, or a TMA store
 STORE = re.compile(r"\*p\.\w+ = |p\.\w+\[[^\]]*\] = |atomic\w+\(p\.|st\.global|cp\.async\.bulk\.tensor\.\dd\.global|__stcs|__stwt")
+LOAD = re.compile(r"__ldg\(|ld\.global|tma_load_\dd\w*\(|load_2d<")
 
 
 def kernels():
@@ -28,15 +30,15 @@ def kernels():
             yield os.path.basename(path), m.group(1), text[start:i]
 
 
-def test_no_global_store_precedes_the_dependency_wait():
+def test_no_global_access_precedes_the_dependency_wait():
     seen = 0
     for path, name, body in kernels():
         wait = WAIT.search(body)
         if wait is None:      # not launched as a programmatic dependent
             continue
         seen += 1
-        early = STORE.search(body[:wait.start()])
-        assert early is None, f"{path}: {name} stores before its dependency wait: {body[early.start():early.start() + 60]!r}"
+        early = STORE.search(body[:wait.start()]) or LOAD.search(body[:wait.start()])
+        assert early is None, f"{path}: {name} touches memory before its dependency wait: {body[early.start():early.start() + 60]!r}"
     assert seen >= 8
 
 
